@@ -437,11 +437,24 @@ struct Purifier {
   int last_iterations = 0;
   double *pin = nullptr;  // kSp2Len pinned doubles for the purification state
   Purifier(cudaStream_t s, int n_, double *pinned_state) : st(s), n(n_), pin(pinned_state) {
-    X.alloc((size_t)n * n, st);
-    X2.alloc((size_t)n * n, st);
+    const size_t ldx = (size_t)sp2_grid_ld(n);
+    X.alloc(ldx * ldx, st);
+    X2.alloc(ldx * ldx, st);
     scratch.alloc(1024, st);
     bounds.alloc(2, st);
     state.alloc(kSp2Len, st);
+  }
+  // Workspace of the cooperative launches (kernels_sp2.cu) and the barrier's error flag.
+  DevBuf<double> grid_ws;
+  DevBuf<unsigned> grid_count;
+  DevBuf<int> grid_err;
+  void ensure_grid() {
+    if (grid_ws.p) return;
+    grid_ws.alloc(sp2_grid_doubles(n), st);
+    grid_count.alloc(1, st);
+    grid_err.alloc(1, st);
+    CUDA_OK(cudaMemsetAsync(grid_ws.p, 0, sizeof(double) * sp2_grid_doubles(n), st));
+    CUDA_OK(cudaMemsetAsync(grid_err.p, 0, sizeof(int), st));
   }
   // fp32 iterate of the mixed-precision purification: X, its tf32 split, X^2 (ld x ld)
   int ld = 0;
@@ -566,60 +579,84 @@ struct Purifier {
     if (e) CUDA_OK(cudaMemsetAsync(i8err.p, 0, sizeof(int), st));
     return e;
   }
+  // A whole purification as one cooperative launch on the FP64 tensor cores.
+  bool project_grid(const double *F, int n_occ, double w, const Sp2Rule &rule, bool refine, double *P) {
+    const int mode = refine && n > kSp2BoundsMax ? 2 : refine ? 1 : 0;
+    if (mode == 2) bounds_of(F, true);
+    {
+      Stage g_(st, "sp2_grid");
+      launch_sp2_purify(st, n, F, mode, (double)n_occ, w, rule, X.p, X2.p, P, grid_ws.p, bounds.p, state.p,
+                        grid_count.p, grid_err.p);
+    }
+    int *bad = reinterpret_cast<int *>(pin + kSp2Len);
+    CUDA_OK(cudaMemcpyAsync(pin, state.p, kSp2Len * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CUDA_OK(cudaMemcpyAsync(bad, grid_err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CUDA_OK(cudaStreamSynchronize(st));
+    if (*bad) throw Failure{PM7_ERR_TIMEOUT, "SP2 purification: a grid barrier expired"};
+    last_iterations = (int)pin[kSp2Stop] + 1;
+    return pin[kSp2Ok] != 0.0 && std::fabs(pin[kSp2TrX] - (double)n_occ) <= 1.0e-3;
+  }
+  // The spectral interval of F into `bounds`: Gershgorin, narrowed by Lanczos when refined.
+  void bounds_of(const double *F, bool refine) {
+    if (n <= kSp2BoundsMax) {
+      Stage l_(st, "sp2_bounds");
+      launch_sp2_bounds(st, n, F, refine, grid_ws.p, bounds.p, grid_count.p, grid_err.p);
+      return;
+    }
+    launch_gershgorin(st, n, F, scratch.p, bounds.p);
+    if (!refine) return;
+    Stage l_(st, "sp2_bounds");
+    if (!lz.p) lz.alloc(lanczos_doubles(n), st);
+    launch_lanczos_bounds(st, n, F, lz.p, bounds.p);
+  }
   bool project(const double *F, int n_occ, double w, double *P) {
-    if (tight && !lz.p) lz.alloc(lanczos_doubles(n), st);
+    ensure_grid();
     for (int attempt = 0; attempt < 2; ++attempt) {
       const bool refine = tight && attempt == 0;
-      launch_gershgorin(st, n, F, scratch.p, bounds.p);
-      if (refine) {
-        Stage l_(st, "sp2_bounds");
-        launch_lanczos_bounds(st, n, F, lz.p, bounds.p);
-      }
-      launch_sp2_init(st, n, F, bounds.p, X.p);
       const Sp2Rule rule{1.0e-13 * std::max(1, n_occ), 1.0e-6, kMaxSteps};
-      // Fused steps on the ping-pong pair (X, X2): step s reads the iterate from one and
-      // writes the next, already updated, to the other; its traces come from the previous
-      // step's epilogue (the first from k_sp2_norms).
-      if (!parts.p) parts.alloc(std::max(sp2_parts_doubles(n), 2 * (size_t)sp2_i8_tiles(n) + 8), st);
-      if (i8) {
-        ensure_i8();
-        launch_sp2_digits(st, n, X.p, dig0.p, nullptr, -1, i8err.p);
-      }
-      const char *stage = i8 ? "sp2_square_i8" : "sp2_square_gemm";
-      last_iterations = run_chunks(
-          [&](int s) {
-            if (s == 0) launch_sp2_norms(st, n, X.p, state.p, parts.p);
-            launch_sp2_decide(st, (double)n_occ, state.p, parts.p, s, rule);
-            Stage g_(st, stage);
-            const double *in = s % 2 == 0 ? X.p : X2.p;
-            double *out = s % 2 == 0 ? X2.p : X.p;
-            if (i8)
-              launch_sp2_step_i8(st, n, dmap[2 * (s % 2)], dmap[2 * (s % 2) + 1], in, out,
-                                 s % 2 == 0 ? dig1.p : dig0.p, state.p, parts.p, s, i8err.p);
-            else
-              launch_sp2_step(st, n, in, out, state.p, parts.p, s);
-          },
-          stage, hint64);
-      bool ok = pin[kSp2Ok] != 0.0;
-      if (i8 && i8_status() != 0) ok = false;
-      // an idempotent X whose trace is not n_occ is a wrong projector (degenerate frontier)
-      if (ok && std::fabs(pin[kSp2TrX] - (double)n_occ) > 1.0e-3) ok = false;
-      if (ok) {
-        const int stop = (int)pin[kSp2Stop];  // the iterate after the last step is in its output
-        launch_scale(st, (size_t)n * n, w, stop % 2 == 0 ? X2.p : X.p, P);
-        return true;
-      }
+      const bool ok = i8 ? project_i8(F, n_occ, w, rule, refine, P) : project_grid(F, n_occ, w, rule, refine, P);
+      if (ok) return true;
       if (!refine) return false;
       tight = false;  // the refined interval missed part of the spectrum: Gershgorin from now on
     }
     return false;
   }
+  // Fused steps on the ping-pong pair (X, X2): step s reads the iterate from one and writes the
+  // next, already updated, to the other; its traces come from the previous step's epilogue (the
+  // first from k_sp2_norms).
+  bool project_i8(const double *F, int n_occ, double w, const Sp2Rule &rule, bool refine, double *P) {
+    bounds_of(F, refine);
+    launch_sp2_init(st, n, F, bounds.p, X.p);
+    if (!parts.p) parts.alloc(sp2_parts_doubles(n), st);
+    ensure_i8();
+    launch_sp2_digits(st, n, X.p, dig0.p, nullptr, -1, i8err.p);
+    last_iterations = run_chunks(
+        [&](int s) {
+          if (s == 0) launch_sp2_norms(st, n, X.p, state.p, parts.p);
+          launch_sp2_decide(st, (double)n_occ, state.p, parts.p, s, rule);
+          Stage g_(st, "sp2_square_i8");
+          const double *in = s % 2 == 0 ? X.p : X2.p;
+          double *out = s % 2 == 0 ? X2.p : X.p;
+          launch_sp2_step_i8(st, n, dmap[2 * (s % 2)], dmap[2 * (s % 2) + 1], in, out, s % 2 == 0 ? dig1.p : dig0.p,
+                             state.p, parts.p, s, i8err.p);
+        },
+        "sp2_square_i8", hint64);
+    int bad = 0;
+    CUDA_OK(cudaMemcpyAsync(&bad, grid_err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    bool ok = pin[kSp2Ok] != 0.0;
+    if (i8_status() != 0) ok = false;  // (synchronises)
+    if (bad) throw Failure{PM7_ERR_TIMEOUT, "SP2 bounds: a grid barrier expired"};
+    // an idempotent X whose trace is not n_occ is a wrong projector (degenerate frontier)
+    if (!ok || std::fabs(pin[kSp2TrX] - (double)n_occ) > 1.0e-3) return false;
+    const int stop = (int)pin[kSp2Stop];  // the iterate after the last step is in its output
+    launch_scale(st, (size_t)n * n, w, stop % 2 == 0 ? X2.p : X.p, P);
+    return true;
+  }
 };
 
 // The fp64 SP2 squarings run on the integer tensor cores (kernels_i8.cu) from kI8MinN orbitals
-// up, on the DMMA GEMM below (the two are level at ~600 orbitals: 0.051 ms per squaring at
-// 600, 0.224 against 0.314 ms at 2,004, 4.2 against 6.9 ms at 6,000); PM7_SP2_GEMM=dmma|i8
-// forces one.
+// up, on the FP64 tensor cores in one cooperative launch below (kernels_sp2.cu);
+// PM7_SP2_GEMM=dmma|i8 forces one.
 constexpr int kI8MinN = 768;
 static bool use_i8_sp2(int n) {
   const char *env = std::getenv("PM7_SP2_GEMM");

@@ -242,19 +242,26 @@ constexpr int kLzSteps = 16;
 size_t lanczos_doubles(int n);
 void launch_lanczos_bounds(cudaStream_t st, int n, const double *F, double *lz, double *bounds);
 void launch_sp2_reset(cudaStream_t st, double *state);
-void launch_sp2_square(cudaStream_t st, int n, const double *X, double *X2, const double *state, int step);
-void launch_sp2_trace(cudaStream_t st, int n, const double *X, const double *X2, double n_occ, double *state, int step,
-                      Sp2Rule rule);
-void launch_sp2_update(cudaStream_t st, int n, double *X, const double *X2, const double *state, int step);
 // The fused SP2 iteration on a ping-pong pair: launch_sp2_norms gives the starting iterate's
 // trace partials; per step, launch_sp2_decide turns the current partials into the branch and
-// the stopping rule, and launch_sp2_step writes the next iterate Y = X^2 or 2X - X^2 (the
-// squaring's epilogue applies the branch) with its own partials. `parts` holds
-// sp2_parts_doubles(n) doubles.
+// the stopping rule, and the squaring (launch_sp2_step_i8) writes the next iterate
+// Y = X^2 or 2X - X^2 with its own partials. `parts` holds sp2_parts_doubles(n) doubles.
 size_t sp2_parts_doubles(int n);
 void launch_sp2_norms(cudaStream_t st, int n, const double *X, double *state, double *parts);
 void launch_sp2_decide(cudaStream_t st, double n_occ, double *state, const double *parts, int step, Sp2Rule rule);
-void launch_sp2_step(cudaStream_t st, int n, const double *X, double *Y, double *state, double *parts, int step);
+// A whole purification in one cooperative launch, and its spectral bounds alone
+// (kernels_sp2.cu). F is n x n; x0, x1 are sp2_grid_ld(n)^2; ws sp2_grid_doubles(n), zeroed once; P becomes
+// w times the projector; lanczos 1: narrowed bounds, 0: Gershgorin, 2: those in `bounds`. The
+// last step's Sp2State is left in state; count is a scratch counter; *error becomes 1 when a
+// grid barrier expired. launch_sp2_bounds takes n up to kSp2BoundsMax.
+constexpr int kSp2BoundsMax = 9400;  // three Lanczos vectors in one CTA's shared memory
+int sp2_grid_ld(int n);
+size_t sp2_grid_doubles(int n);
+void launch_sp2_bounds(cudaStream_t st, int n, const double *F, bool lanczos, double *ws, double *bounds,
+                       unsigned *count, int *error);
+void launch_sp2_purify(cudaStream_t st, int n, const double *F, int lanczos, double n_occ, double w, Sp2Rule rule,
+                       double *x0, double *x1, double *P, double *ws, double *bounds, double *state, unsigned *count,
+                       int *error);
 }
 
 namespace pm7 {

@@ -291,30 +291,15 @@ static inline int sym_tiles(int n) {
   return t;
 }
 
-// The fused SP2 step of a symmetric n x n product (launch_sp2_step): parts != null makes
-// the tiles apply the update chosen in state[kSp2Square] and write the 64 x 64 block trace
-// partials; the first CTA records their count in state[kSp2Parts].
-__device__ __forceinline__ Sp2Fuse sp2_fuse(int n, const double *x, double *state, double *parts) {
-  if (!parts) return Sp2Fuse{nullptr, false, nullptr, 1.0};
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const int t64 = (n + 63) / 64;
-    state[kSp2Parts] = (double)(t64 * (t64 + 1) / 2);
-  }
-  return Sp2Fuse{x, state[kSp2Square] != 0.0, parts, 1.0};
-}
-
 // Symmetric n x n product on 64x64 tiles of the lower triangle (four CTAs per SM): more,
 // smaller tiles than k_gemm_sym, the faster shape when 128x64 tiles leave SMs idle.
 __global__ void __launch_bounds__(128, 4) k_gemm_sym64(int n, int K, double alpha, const double *__restrict__ A,
                                                        int lda, const double *__restrict__ B, int ldb,
-                                                       double *__restrict__ C, int ldc, double *__restrict__ sp2,
-                                                       int step, double *__restrict__ parts) {
+                                                       double *__restrict__ C, int ldc) {
   extern __shared__ __align__(16) double gemm_smem[];
-  if (!sp2_active(sp2, step)) return;
   int t = blockIdx.x, r = 0;
   while ((r + 1) * (r + 2) / 2 <= t) ++r;
-  gemm_tile_t<BM, BN>(gemm_smem, r, t - r * (r + 1) / 2, n, n, K, alpha, A, lda, B, ldb, C, ldc, 1,
-                      sp2_fuse(n, A, sp2, parts));
+  gemm_tile_t<BM, BN>(gemm_smem, r, t - r * (r + 1) / 2, n, n, K, alpha, A, lda, B, ldb, C, ldc, 1);
 }
 
 // Symmetric n x n product over the enumerated lower-triangle tiles (row block r holds
@@ -322,10 +307,8 @@ __global__ void __launch_bounds__(128, 4) k_gemm_sym64(int n, int K, double alph
 template <int TBK, int TST>
 __global__ void __launch_bounds__(128, 2) k_gemm_sym(int n, int K, double alpha, const double *__restrict__ A,
                                                      int lda, const double *__restrict__ B, int ldb,
-                                                     double *__restrict__ C, int ldc, double *__restrict__ sp2,
-                                                     int step, double *__restrict__ parts) {
+                                                     double *__restrict__ C, int ldc) {
   extern __shared__ __align__(16) double gemm_smem[];
-  if (!sp2_active(sp2, step)) return;  // an SP2 step after the purification stopped
   const int cols = (n + SYM_BN - 1) / SYM_BN;
   int t = blockIdx.x, r = 0;
   for (;; ++r) {
@@ -333,8 +316,7 @@ __global__ void __launch_bounds__(128, 2) k_gemm_sym(int n, int K, double alpha,
     if (t < nc) break;
     t -= nc;
   }
-  gemm_tile_t<SYM_BM, SYM_BN, TBK, TST>(gemm_smem, r, t, n, n, K, alpha, A, lda, B, ldb, C, ldc, 1,
-                                        sp2_fuse(n, A, sp2, parts));
+  gemm_tile_t<SYM_BM, SYM_BN, TBK, TST>(gemm_smem, r, t, n, n, K, alpha, A, lda, B, ldb, C, ldc, 1);
 }
 
 // Grouped over molecules: item = one 64x64 tile of one molecule's product.
@@ -412,38 +394,32 @@ void launch_gemm_tn(cudaStream_t st, int M, int N, int K, double alpha, const do
 // Symmetric product C = alpha A^T B (n x n, inner dimension K) on the tile shape the
 // autotuner picked for this size: 0 = 128x64 (k_gemm_sym, 16-deep slabs, three stages),
 // 1 = 64x64 (k_gemm_sym64), 2 = 128x64 with 32-deep slabs in two stages. All give the same
-// bits: every element is the same chain of DMMA steps over k in the same order. With
-// `parts` the product is the fused SP2 step (sp2_fuse).
+// bits: every element is the same chain of DMMA steps over k in the same order.
 static void launch_sym(cudaStream_t st, const char *what, int n, int K, double alpha, const double *A, int lda,
-                       const double *B, int ldb, double *C, int ldc, double *sp2, int step, double *parts = nullptr) {
+                       const double *B, int ldb, double *C, int ldc) {
   gemm_smem_attr();
   const int bucket = ((n + 255) / 256) * 256;
   autotune(st, std::string(what) + "|n" + std::to_string(bucket), 3, [&](int v) {
     if (v == 0) {
-      k_gemm_sym<BK, STAGES><<<sym_tiles(n), 128, SYM_SMEM, st>>>(n, K, alpha, A, lda, B, ldb, C, ldc, sp2, step,
-                                                                  parts);
+      k_gemm_sym<BK, STAGES><<<sym_tiles(n), 128, SYM_SMEM, st>>>(n, K, alpha, A, lda, B, ldb, C, ldc);
     } else if (v == 1) {
       const int t = (n + BM - 1) / BM;
-      k_gemm_sym64<<<t * (t + 1) / 2, 128, GEMM_SMEM, st>>>(n, K, alpha, A, lda, B, ldb, C, ldc, sp2, step, parts);
+      k_gemm_sym64<<<t * (t + 1) / 2, 128, GEMM_SMEM, st>>>(n, K, alpha, A, lda, B, ldb, C, ldc);
     } else {
-      k_gemm_sym<32, 2><<<sym_tiles(n), 128, SYM_SMEM_K32, st>>>(n, K, alpha, A, lda, B, ldb, C, ldc, sp2, step,
-                                                                  parts);
+      k_gemm_sym<32, 2><<<sym_tiles(n), 128, SYM_SMEM_K32, st>>>(n, K, alpha, A, lda, B, ldb, C, ldc);
     }
     note_launch();
   });
 }
 
-size_t sp2_parts_doubles(int n) {
-  const int t = (n + BM - 1) / BM;
-  return 2 * (size_t)std::max(std::max(sym_tiles(n), t * (t + 1) / 2), 296) + 8;
-}
+size_t sp2_parts_doubles(int n) { return 2 * (size_t)std::max(sp2_i8_tiles(n), 296) + 8; }
 
 void launch_density(cudaStream_t st, int n, int k, double w, const double *V, int ldv, double *P) {
   if (k == 0) {
     cudaMemsetAsync(P, 0, sizeof(double) * (size_t)n * n, st);
     return;
   }
-  launch_sym(st, "density_sym", n, k, w, V, ldv, V, ldv, P, n, nullptr, 0);
+  launch_sym(st, "density_sym", n, k, w, V, ldv, V, ldv, P, n);
 }
 
 // ---------------------------------------------------------------------------
@@ -876,37 +852,6 @@ __global__ void k_sp2_init(int n, const double *__restrict__ F, const double *__
   }
 }
 
-// Traces of X and X^2 and the SP2 branch: state[0] = tr X, state[1] = tr X^2,
-// state[2] = 1 when squaring brings the trace closer to n_occ, state[3] = tr X - tr X^2;
-// then the stopping rule.
-__global__ void k_sp2_trace(int n, const double *__restrict__ X, const double *__restrict__ X2, double n_occ,
-                            double *__restrict__ state, int step, Sp2Rule rule) {
-  if (!sp2_active(state, step)) return;
-  double a = 0.0, b = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    a += X[(size_t)i * n + i];
-    b += X2[(size_t)i * n + i];
-  }
-  a = block_sum<256>(a);
-  b = block_sum<256>(b);
-  if (threadIdx.x == 0) {
-    state[kSp2TrX] = a;
-    state[kSp2TrX2] = b;
-    state[kSp2Square] = fabs(b - n_occ) < fabs(2.0 * a - b - n_occ) ? 1.0 : 0.0;
-    state[kSp2Err] = a - b;
-    sp2_control(state, step, a - b, rule);
-  }
-}
-
-// X <- X^2 or 2X - X^2 according to state[2].
-__global__ void k_sp2_update(size_t len, double *__restrict__ X, const double *__restrict__ X2,
-                             const double *__restrict__ state, int step) {
-  if (!sp2_active(state, step)) return;
-  const bool square = state[kSp2Square] != 0.0;
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < len; e += (size_t)gridDim.x * blockDim.x)
-    X[e] = square ? X2[e] : 2.0 * X[e] - X2[e];
-}
-
 // tr X and |X|_F^2 (= tr X^2 for symmetric X) of the starting iterate, per-block partials in
 // the layout of the fused step's (parts[2 b], parts[2 b + 1]); the count to state[kSp2Parts].
 __global__ void k_sp2_norms(int n, const double *__restrict__ X, double *__restrict__ state,
@@ -988,14 +933,6 @@ void launch_sp2_reset(cudaStream_t st, double *state) {
   note_launch();
 }
 
-void launch_sp2_square(cudaStream_t st, int n, const double *X, double *X2, const double *state, int step) {
-  launch_sym(st, "sp2_square", n, n, 1.0, X, n, X, n, X2, n, const_cast<double *>(state), step);
-}
-
-void launch_sp2_step(cudaStream_t st, int n, const double *X, double *Y, double *state, double *parts, int step) {
-  launch_sym(st, "sp2_square", n, n, 1.0, X, n, X, n, Y, n, state, step, parts);
-}
-
 void launch_sp2_norms(cudaStream_t st, int n, const double *X, double *state, double *parts) {
   k_sp2_norms<<<296, 256, 0, st>>>(n, X, state, parts);
   note_launch();
@@ -1003,17 +940,6 @@ void launch_sp2_norms(cudaStream_t st, int n, const double *X, double *state, do
 
 void launch_sp2_decide(cudaStream_t st, double n_occ, double *state, const double *parts, int step, Sp2Rule rule) {
   k_sp2_decide<<<1, 256, 0, st>>>(n_occ, state, parts, step, rule);
-  note_launch();
-}
-
-void launch_sp2_trace(cudaStream_t st, int n, const double *X, const double *X2, double n_occ, double *state, int step,
-                      Sp2Rule rule) {
-  k_sp2_trace<<<1, 256, 0, st>>>(n, X, X2, n_occ, state, step, rule);
-  note_launch();
-}
-
-void launch_sp2_update(cudaStream_t st, int n, double *X, const double *X2, const double *state, int step) {
-  k_sp2_update<<<RED_BLOCKS * 2, 256, 0, st>>>((size_t)n * n, X, X2, state, step);
   note_launch();
 }
 
