@@ -555,19 +555,17 @@ struct Purifier {
   bool tight = true;
 
   // FP64-accuracy squarings on the integer tensor cores (int8 digit planes, kernels_i8.cu):
-  // two plane sets, read and written alternately with X and X2, and their tensor maps.
+  // two plane sets, read and written alternately with X and X2.
   bool i8 = false;
   DevBuf<int8_t> dig0, dig1;
   DevBuf<int> i8err;
-  alignas(64) unsigned char dmap[4][128];
   void ensure_i8() {
     if (dig0.p) return;
     dig0.alloc(sp2_i8_digit_bytes(n), st);
     dig1.alloc(sp2_i8_digit_bytes(n), st);
     i8err.alloc(1, st);
     CUDA_OK(cudaMemsetAsync(i8err.p, 0, sizeof(int), st));
-    if (!make_digit_maps(dig0.p, n, dmap[0], dmap[1]) || !make_digit_maps(dig1.p, n, dmap[2], dmap[3]))
-      throw Failure{PM7_ERR_CUDA, "cuTensorMapEncodeTiled failed"};
+    for (DevBuf<int8_t> *d : {&dig0, &dig1}) CUDA_OK(cudaMemsetAsync(d->p, 0, sp2_i8_digit_bytes(n), st));
   }
   // 1: a pipeline wait expired (raised), 2: an iterate element left the digits' range (the
   // purification is treated as failed); the flag is cleared.
@@ -637,8 +635,7 @@ struct Purifier {
           Stage g_(st, "sp2_square_i8");
           const double *in = s % 2 == 0 ? X.p : X2.p;
           double *out = s % 2 == 0 ? X2.p : X.p;
-          launch_sp2_step_i8(st, n, dmap[2 * (s % 2)], dmap[2 * (s % 2) + 1], in, out, s % 2 == 0 ? dig1.p : dig0.p,
-                             state.p, parts.p, s, i8err.p);
+          launch_sp2_step_i8(st, n, s % 2 == 0 ? dig0.p : dig1.p, in, out, s % 2 == 0 ? dig1.p : dig0.p, state.p, parts.p, s, i8err.p);
         },
         "sp2_square_i8", hint64);
     int bad = 0;
@@ -1979,10 +1976,9 @@ pm7_status pm7_stage_sp2_step_i8(int32_t n, const double *x, int32_t square, dou
     launch_sp2_reset(st, state.p);
     const double sq = square ? 1.0 : 0.0;
     CUDA_OK(cudaMemcpyAsync(state.p + kSp2Square, &sq, sizeof(double), cudaMemcpyHostToDevice, st));
+    CUDA_OK(cudaMemsetAsync(dig0.p, 0, sp2_i8_digit_bytes(n), st));
     launch_sp2_digits(st, n, X.p, dig0.p, nullptr, -1, err.p);
-    alignas(64) unsigned char map_a[128], map_b[128];
-    if (!make_digit_maps(dig0.p, n, map_a, map_b)) throw Failure{PM7_ERR_CUDA, "cuTensorMapEncodeTiled failed"};
-    launch_sp2_step_i8(st, n, map_a, map_b, X.p, Y.p, dig1.p, state.p, parts.p, 0, err.p);
+    launch_sp2_step_i8(st, n, dig0.p, X.p, Y.p, dig1.p, state.p, parts.p, 0, err.p);
     std::vector<double> ph(2 * (size_t)tiles);
     int e = 0;
     CUDA_OK(cudaMemcpyAsync(&e, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));

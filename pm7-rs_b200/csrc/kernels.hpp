@@ -186,21 +186,17 @@ struct Sp2Rule {
 
 namespace pm7 {
 // FP64-accuracy SP2 squarings on the tcgen05 integer tensor cores (kernels_i8.cu): the
-// iterate in fp64 (n x n) and as eight int8 digit planes (sp2_i8_digit_bytes(n) bytes, rows of
-// sp2_i8_ld(n) bytes) whose two tensor maps (128-byte opaque CUtensorMap each) come from
-// make_digit_maps. launch_sp2_step_i8 is the fused step of launch_sp2_step (same state, step
-// and partial protocol) reading x_in and its planes, writing x_out and its planes; `error`:
-// 1 a pipeline wait expired, 2 an element left the digits' range. launch_sp2_digits splits X
-// into planes (step < 0: unconditionally; else only while that step is active).
-int sp2_i8_ld(int n);
+// iterate in fp64 (n x n) and as eight int8 digit planes (sp2_i8_digit_bytes(n) bytes, zeroed
+// once, 16-byte aligned). launch_sp2_step_i8 is one fused step (state, step index and trace partials,
+// 2 sp2_i8_tiles(n) doubles; the next decision reads them) and splits its output; *error becomes
+// 1 when a pipeline wait expired, 2 when an element left the digits' range. launch_sp2_digits
+// splits X (step < 0: always; else only while the purification runs).
 size_t sp2_i8_digit_bytes(int n);
 int sp2_i8_tiles(int n);
-bool make_digit_maps(const int8_t *dig, int n, void *map_a, void *map_b);
-void prepare_i8_kernels();
 void launch_sp2_digits(cudaStream_t st, int n, const double *X, int8_t *dig, const double *state, int step,
                        int *error);
-void launch_sp2_step_i8(cudaStream_t st, int n, const void *map_a, const void *map_b, const double *x_in,
-                        double *x_out, int8_t *dig_out, double *state, double *parts, int step, int *error);
+void launch_sp2_step_i8(cudaStream_t st, int n, const int8_t *dig, const double *x_in, double *x_out, int8_t *dig_out,
+                        double *state, double *parts, int step, int *error);
 }  // namespace pm7
 
 namespace pm7 {
