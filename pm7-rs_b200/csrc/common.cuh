@@ -27,6 +27,14 @@ __device__ __forceinline__ double block_sum(double v) {
   return s;
 }
 
+// The power of two that brings a largest element `big` into [1, 2); 1 for zero, subnormal or
+// non-finite ones.
+__device__ __forceinline__ double tri_scale(double big) {
+  const int e = __double2hiint(big) & 0x7ff00000;
+  if (e == 0 || e >= 0x7fe00000) return 1.0;
+  return __hiloint2double(0x7fe00000 - e, 0);
+}
+
 // One step of the device-side SP2 stopping rule (Sp2State, Sp2Rule in kernels.hpp), run by
 // a single thread after the step's traces are in state: records the step's error, and on
 // convergence, the rounding floor, a non-finite error or the step cap sets

@@ -366,7 +366,6 @@ static bool use_jacobi(int n) {
   return env && std::strcmp(env, "jacobi") == 0 && n <= kJacobiMax;
 }
 
-constexpr int kOwnEigvalsMax = 511;  // eigenvalues alone: the cluster tridiagonalisation up to here
 
 struct Diag {
   DeviceContext &ctx;
@@ -378,7 +377,7 @@ struct Diag {
   DevBuf<int> info;
   DevBuf<JacobiJob> job;
   double *slot = nullptr;
-  bool warm = false, pending = false;
+  bool warm = false, pending = false, own_values = false;
   int *pin;  // pinned copy of the Jacobi status
   Diag(DeviceContext &ctx, int n_, double *probe, int *pinned_info)
       : ctx(ctx), st(ctx.stream), n(n_), jac(use_jacobi(n_)), pin(pinned_info) {
@@ -406,18 +405,23 @@ struct Diag {
     pending = true;
   }
   // Eigenvalues of A into eps(); A keeps its contents unless the solver is Jacobi or
-  // cuSOLVER (which leave eigenvectors). Up to kOwnEigvalsMax the values come from the
-  // repo's cluster tridiagonalisation and Sturm multisection.
+  // cuSOLVER (which leave eigenvectors). Up to kTriGridMax the values come from the repo's
+  // tridiagonalisations and Sturm multisection.
   void values(double *A) {
     const char *env = std::getenv("PM7_DENSITY_SOLVER");
     const bool library_only = env && std::strcmp(env, "syevd") == 0;
-    if (jac || library_only || n > kOwnEigvalsMax) {
+    if (jac || library_only || n > kTriGridMax) {
       solve(A, false);
       return;
     }
-    eigvals_device(st, {EigvalsRequest{A, n, n, lib->eps.p}}, ctx.eig_scratch);
+    eigvals_device(st, {EigvalsRequest{A, n, n, lib->eps.p}}, ctx.eig_scratch, true);
+    own_values = true;
   }
   void check() {
+    if (own_values) {
+      own_values = false;
+      eigvals_check(st, ctx.eig_scratch);
+    }
     if (!pending) return;
     pending = false;
     if (*pin != 0)
@@ -976,15 +980,25 @@ static void run_rhf(DeviceContext &ctx, const DeviceParams &P, DeviceMolecule &D
   out.n_occ = n_occ;
 }
 
-void eigvals_device(cudaStream_t st, const std::vector<EigvalsRequest> &req, EigvalsScratch &scr) {
+void eigvals_check(cudaStream_t st, EigvalsScratch &scr) {
+  if (!scr.expired) return;
+  int e = 0;
+  CUDA_OK(cudaMemcpyAsync(&e, scr.expired, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CUDA_OK(cudaStreamSynchronize(st));
+  if (!e) return;
+  CUDA_OK(cudaMemsetAsync(scr.expired, 0, sizeof(int), st));
+  throw Failure{PM7_ERR_TIMEOUT, "eigenvalue solve: a grid barrier expired"};
+}
+
+void eigvals_device(cudaStream_t st, const std::vector<EigvalsRequest> &req, EigvalsScratch &scr, bool whole_gpu) {
   if (req.empty()) return;
-  std::map<int, std::vector<int>> groups;  // cluster size -> requests
+  std::map<int, std::vector<int>> groups;  // cluster size (0: the whole GPU) -> requests
   size_t work = 0;
   for (size_t i = 0; i < req.size(); ++i) {
     const int n = req[i].n;
     if (!eigvals_supported(n) || req[i].ld < n)
       throw Failure{PM7_ERR_INVALID_INPUT, "eigenvalue solve: order " + std::to_string(n) + " not supported"};
-    groups[tridiag_cluster_size(n)].push_back((int)i);
+    groups[whole_gpu && tridiag_grid_supported(n) ? 0 : tridiag_cluster_size(n)].push_back((int)i);
     work += (eigvals_work_doubles(n) + 31) / 32 * 32;
   }
   // per group: its tasks, then its prefix sums (int), in one uploaded block
@@ -1044,10 +1058,46 @@ void eigvals_device(cudaStream_t st, const std::vector<EigvalsRequest> &req, Eig
   std::memcpy(scr.pinned, meta.data(), meta.size());
   CUDA_OK(cudaMemcpyAsync(scr.meta, scr.pinned, meta.size(), cudaMemcpyHostToDevice, st));
   CUDA_OK(cudaEventRecord(scr.uploaded, st));
-  for (const G &g : gs) {
-    const cudaError_t err =
-        launch_eigvals(st, reinterpret_cast<const EigvalsTask *>(scr.meta + g.tasks_off), g.count, g.c, g.max_n,
-                       reinterpret_cast<const int *>(scr.meta + g.prefix_off), g.total);
+  // The groups side by side (a group's time is that of its largest matrix, on few SMs): the first on
+  // st, each other on a stream of its own that st forks and joins.
+  const size_t sides = gs.size() - 1;
+  if (sides > 0) {
+    while (scr.side.size() < sides) {
+      EigvalsScratch::Side s{};
+      CUDA_OK(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
+      scr.side.push_back(s);
+      CUDA_OK(cudaEventCreateWithFlags(&scr.side.back().done, cudaEventDisableTiming));
+    }
+    if (!scr.forked) CUDA_OK(cudaEventCreateWithFlags(&scr.forked, cudaEventDisableTiming));
+    CUDA_OK(cudaEventRecord(scr.forked, st));
+    for (size_t q = 0; q < sides; ++q) CUDA_OK(cudaStreamWaitEvent(scr.side[q].st, scr.forked, 0));
+  }
+  const cudaStream_t main_st = st;
+  for (size_t gi = gs.size(); gi-- > 0;) {  // the largest cluster size first
+    const G &g = gs[gi];
+    const cudaStream_t st = gi + 1 == gs.size() ? main_st : scr.side[gi].st;
+    const EigvalsTask *tasks = reinterpret_cast<const EigvalsTask *>(scr.meta + g.tasks_off);
+    const int *prefix = reinterpret_cast<const int *>(scr.meta + g.prefix_off);
+    cudaError_t err = cudaSuccess;
+    if (g.c == 0) {
+      if (!scr.expired) {
+        CUDA_OK(cudaMallocAsync((void **)&scr.expired, sizeof(int), st));
+        CUDA_OK(cudaMemsetAsync(scr.expired, 0, sizeof(int), st));
+      }
+      const EigvalsTask *host = reinterpret_cast<const EigvalsTask *>(meta.data() + g.tasks_off);
+      {
+        Stage s_(st, "tridiagonalise");
+        for (int q = 0; q < g.count && err == cudaSuccess; ++q) err = launch_tridiag_grid(st, host[q], scr.expired);
+      }
+      Stage s_(st, "tridiagonal_values");
+      if (err == cudaSuccess) err = launch_tri_eigs(st, tasks, g.count, prefix, g.total);
+    } else {
+      err = launch_eigvals(st, tasks, g.count, g.c, g.max_n, prefix, g.total);
+    }
+    if (st != main_st) {
+      CUDA_OK(cudaEventRecord(scr.side[gi].done, st));
+      CUDA_OK(cudaStreamWaitEvent(main_st, scr.side[gi].done, 0));
+    }
     if (err != cudaSuccess) throw Failure{PM7_ERR_CUDA, std::string("eigenvalue solve: ") + cudaGetErrorString(err)};
   }
 }
@@ -1194,22 +1244,31 @@ static void run_uhf(DeviceContext &ctx, const DeviceParams &P, DeviceMolecule &D
   CUDA_OK(cudaMemcpyAsync(sc, dscal.p, sizeof(double) * 3, cudaMemcpyDeviceToHost, st));
   CUDA_OK(cudaStreamSynchronize(st));
   out.electronic_ev = 0.5 * (sc[0] + sc[1] + sc[2]);
-  out.Va.alloc(nn, st);
-  out.Vb.alloc(nn, st);
+  if (o.want_matrices) {
+    out.Va.alloc(nn, st);
+    out.Vb.alloc(nn, st);
+  }
+  // the levels, and the orbitals when matrices are returned
+  const bool vectors = o.want_matrices != 0;
+  auto levels = [&](Diag &e, double *A) {
+    Stage s_(st, "eigensolve");
+    if (vectors) e.solve(A);
+    else e.values(A);
+  };
   if (guard.shift > 0.0) {
     CUDA_OK(cudaMemcpyAsync(Ua.p, Fa.p, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st));
-    { Stage s_(st, "eigensolve"); eig.solve(Ua.p); }
+    levels(eig, Ua.p);
     out.eps_a.resize(n);
     CUDA_OK(cudaMemcpyAsync(out.eps_a.data(), eig.eps(), sizeof(double) * n, cudaMemcpyDeviceToHost, st));
   } else if (!diag_a) {
-    { Stage s_(st, "eigensolve"); eig.solve(Ua.p); }
+    levels(eig, Ua.p);
     out.eps_a.resize(n);
     CUDA_OK(cudaMemcpyAsync(out.eps_a.data(), eig.eps(), sizeof(double) * n, cudaMemcpyDeviceToHost, st));
   }
-  CUDA_OK(cudaMemcpyAsync(out.Va.p, Ua.p, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st));
+  if (vectors) CUDA_OK(cudaMemcpyAsync(out.Va.p, Ua.p, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st));
   CUDA_OK(cudaMemcpyAsync(Ub.p, Fb.p, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st));
-  { Stage s_(st, "eigensolve"); eig_b.solve(Ub.p); }
-  CUDA_OK(cudaMemcpyAsync(out.Vb.p, Ub.p, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st));
+  levels(eig_b, Ub.p);
+  if (vectors) CUDA_OK(cudaMemcpyAsync(out.Vb.p, Ub.p, sizeof(double) * nn, cudaMemcpyDeviceToDevice, st));
   out.eps_b.resize(n);
   CUDA_OK(cudaMemcpyAsync(out.eps_b.data(), eig_b.eps(), sizeof(double) * n, cudaMemcpyDeviceToHost, st));
   CUDA_OK(cudaStreamSynchronize(st));

@@ -132,15 +132,32 @@ struct EigvalsScratch {
   size_t meta_cap = 0;  // bytes
   unsigned char *pinned = nullptr;  // host staging of the task table (same capacity)
   cudaEvent_t uploaded = nullptr;   // the last upload from `pinned` has been read
+  int *expired = nullptr;           // device flag: a whole-GPU reduction's barrier wait ran out
+  // streams for the cluster-size groups of one call beside the caller's
+  struct Side {
+    cudaStream_t st = nullptr;
+    cudaEvent_t done = nullptr;
+  };
+  std::vector<Side> side;
+  cudaEvent_t forked = nullptr;
   // stream-ordered release (the owner's stream); the owner calls it before it goes away
   void release(cudaStream_t st) {
     if (uploaded) cudaEventSynchronize(uploaded);
     if (work) cudaFreeAsync(work, st);
     if (meta) cudaFreeAsync(meta, st);
+    if (expired) cudaFreeAsync(expired, st);
     if (pinned) cudaFreeHost(pinned);
     if (uploaded) cudaEventDestroy(uploaded);
+    if (forked) cudaEventDestroy(forked);
+    for (Side &s : side) {  // (their work has been joined to st)
+      if (s.done) cudaEventDestroy(s.done);
+      if (s.st) cudaStreamDestroy(s.st);
+    }
+    side.clear();
+    forked = nullptr;
     work = nullptr;
     meta = pinned = nullptr;
+    expired = nullptr;
     uploaded = nullptr;
     cap = meta_cap = 0;
   }
@@ -239,8 +256,13 @@ struct EigvalsRequest {
 };
 // Eigenvalues only, many matrices at once (kernels_eig.cu): grouped by cluster size, one
 // tridiagonalisation and one Sturm launch per group; workspace from `scr` (grown in
-// stream order as needed). Every order must satisfy eigvals_supported().
-void eigvals_device(cudaStream_t st, const std::vector<EigvalsRequest> &req, EigvalsScratch &scr);
+// stream order as needed). Every order must satisfy eigvals_supported(). whole_gpu: matrices from
+// kTriGridMin up are reduced one after the other by the whole GPU (kernels_trigrid.cu): for callers
+// that wait for them with nothing else to run; eigvals_check then reports an expired barrier after a
+// stream synchronisation.
+void eigvals_device(cudaStream_t st, const std::vector<EigvalsRequest> &req, EigvalsScratch &scr,
+                    bool whole_gpu = false);
+void eigvals_check(cudaStream_t st, EigvalsScratch &scr);
 
 template <class T>
 inline void upload(DevBuf<T> &b, const std::vector<T> &v, cudaStream_t st) {

@@ -285,6 +285,13 @@ int tridiag_cluster_size(int n);
 // Whether order n runs here (order and the per-CTA shared memory it needs); larger
 // matrices go to the library eigensolver.
 bool eigvals_supported(int n);
+// The reduction of one matrix by a cooperative launch over the whole GPU (kernels_trigrid.cu), in
+// place of k_tridiag; orders 2 .. kTriGridMax. *error becomes 1 when a grid barrier expired.
+constexpr int kTriGridMax = 2048;
+bool tridiag_grid_supported(int n);
+cudaError_t launch_tridiag_grid(cudaStream_t st, EigvalsTask t, int *error);
+// The eigenvalues of already tridiagonal tasks (d, e^2, part): the second half of launch_eigvals.
+cudaError_t launch_tri_eigs(cudaStream_t st, const EigvalsTask *tasks, int n_tasks, const int *prefix, int total);
 // All tasks share one cluster size; prefix[t] = sum of the orders of tasks before t,
 // total = sum of all orders (device arrays / values). Returns the launch status.
 cudaError_t launch_eigvals(cudaStream_t st, const EigvalsTask *tasks, int n_tasks, int cluster, int max_n,

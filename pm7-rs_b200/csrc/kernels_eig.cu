@@ -119,9 +119,28 @@ __global__ void __launch_bounds__(THREADS, 1) k_tridiag(const EigvalsTask *__res
     return warp_sum(v);
   };
 
+  // the working copy, scaled by a power of two to a largest element in [1, 2)
+  double big = 0.0;
+  for (int m = warp; m < cnt; m += WARPS)
+    for (int k = lane; k < n; k += 32) big = fmax(big, fabs(T.src[(size_t)(r + m * C) * T.ld + k]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+  if (lane == 0) S.red[warp] = big;
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < WARPS; ++w) big = fmax(big, S.red[w]);
+    S.pt[P_SIG] = big;
+  }
+  cluster.sync();
+  big = lane < C ? cluster.map_shared_rank(S.pt, lane)[P_SIG] : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+  cluster.sync();
+  const double sc = tri_scale(big);
+  if (r == 0 && tid == 0) T.part[3] = 1.0 / sc;
   for (int m = warp; m < cnt; m += WARPS) {
     const int i = r + m * C;
-    for (int k = lane; k < n; k += 32) a[(size_t)i * n + k] = T.src[(size_t)i * T.ld + k];
+    for (int k = lane; k < n; k += 32) a[(size_t)i * n + k] = T.src[(size_t)i * T.ld + k] * sc;
   }
 
   double tau_prev = 0.0;
@@ -317,18 +336,41 @@ __global__ void __launch_bounds__(THREADS, 1) k_tridiag(const EigvalsTask *__res
   }
 }
 
-// Number of eigenvalues of the tridiagonal (d, e^2) below x (Sturm count with a pivot
-// floor, LAPACK dlaebz's recurrence).
-__device__ __forceinline__ int sturm_count(const double *__restrict__ d, const double *__restrict__ e2, int n, double x,
-                                           double pivmin) {
-  double q = d[0] - x;
-  if (fabs(q) < pivmin) q = -pivmin;
-  int c = q < 0.0;
-  for (int i = 1; i < n; ++i) {
-    q = d[i] - x - e2[i - 1] / q;
-    if (fabs(q) < pivmin) q = -pivmin;
-    c += q < 0.0;
+// Number of eigenvalues of the tridiagonal T = (d, e^2) below x, from the leading principal minors
+// of T - x: p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2}, a sign change per negative pivot
+// p_i / p_{i-1}. One dependent FMA per step where the pivots' recurrence (LAPACK dlaebz) needs a
+// division: the launch is a latency chain (14 warps an SM at 2,004 orbitals), 2.65 -> 1.17 ms there,
+// 0.27 -> 0.10 ms at 270. Each step perturbs d and e by a rounding, as the pivots do. The matrix is
+// scaled to elements of at most 2, so eight steps change the pair's scale by less than 1e256 and it
+// is renormalised (exactly) after each eight; a zero minor is a pivot of -1e-22.
+__device__ __forceinline__ int sturm_count(const double *__restrict__ d, const double *__restrict__ e2, int n,
+                                           double x) {
+  double p0 = 1.0, p1 = d[0] - x;
+  if (p1 == 0.0) p1 = -1.0e-22;
+  int c = p1 < 0.0;
+  auto step = [&](double di, double ei) {
+    double p2 = fma(di - x, p1, -ei * p0);
+    if (p2 == 0.0) p2 = -1.0e-22 * p1;
+    c += (__double2hiint(p2) ^ __double2hiint(p1)) < 0;
+    p0 = p1;
+    p1 = p2;
+  };
+  int i = 1;
+  for (; i + 8 <= n; i += 8) {
+    double dd[8], ee[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      dd[q] = d[i + q];
+      ee[q] = e2[i + q - 1];
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) step(dd[q], ee[q]);
+    const int e = max(__double2hiint(p0) & 0x7ff00000, __double2hiint(p1) & 0x7ff00000);
+    const double f = __hiloint2double(0x7fe00000 - e, 0);  // 2^(1023 - e): the larger one to [1, 2)
+    p0 *= f;
+    p1 *= f;
   }
+  for (; i < n; ++i) step(d[i], e2[i - 1]);
   return c;
 }
 
@@ -352,7 +394,7 @@ __global__ void __launch_bounds__(256) k_tri_eigs(const EigvalsTask *__restrict_
     const double tol = 4.0 * 2.220446049250313e-16 * fmax(fabs(lo), fabs(hi)) + pivmin;
     if (hi - lo <= tol) break;
     const double x = lo + (hi - lo) * (double)(lane + 1) * (1.0 / 33.0);
-    const int cnt = sturm_count(d, e2, n, x, pivmin);
+    const int cnt = sturm_count(d, e2, n, x);
     const unsigned above = __ballot_sync(0xffffffffu, cnt > k);
     const int f = above ? __ffs(above) - 1 : 32;
     const double xl = __shfl_sync(0xffffffffu, x, f > 0 ? f - 1 : 0);
@@ -360,7 +402,7 @@ __global__ void __launch_bounds__(256) k_tri_eigs(const EigvalsTask *__restrict_
     if (f > 0) lo = xl;
     if (f < 32) hi = xh;
   }
-  if (lane == 0) T.eps[k] = 0.5 * (lo + hi);
+  if (lane == 0) T.eps[k] = 0.5 * (lo + hi) * T.part[3];
 }
 
 constexpr int kSmemMax = 232448;  // opt-in shared memory per CTA on sm_100a (227 KB)
@@ -448,6 +490,10 @@ cudaError_t launch_eigvals(cudaStream_t st, const EigvalsTask *tasks, int n_task
   cudaError_t err = cudaLaunchKernelEx(&cfg, k_tridiag, tasks, cluster, max_n, rmax);
   note_launch();
   if (err != cudaSuccess) return err;
+  return launch_tri_eigs(st, tasks, n_tasks, prefix, total);
+}
+
+cudaError_t launch_tri_eigs(cudaStream_t st, const EigvalsTask *tasks, int n_tasks, const int *prefix, int total) {
   const int threads = 256, warps_per_block = threads / 32;
   k_tri_eigs<<<(total + warps_per_block - 1) / warps_per_block, threads, 0, st>>>(tasks, prefix, n_tasks, total);
   note_launch();
