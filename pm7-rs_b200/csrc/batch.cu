@@ -11,6 +11,7 @@
 // serves a fixed batch and a continuous request stream. Every per-molecule decision is
 // taken on the device from the molecule's MolCtl; the host only rebuilds the work lists
 // and reads one done-flag per molecule per iteration.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <cusolverDn.h>
 
@@ -32,6 +33,8 @@
 #include "common.cuh"
 #include "gradient.cuh"
 #include "engine_internal.hpp"
+
+namespace cg = cooperative_groups;
 
 namespace pm7 {
 
@@ -524,11 +527,15 @@ __global__ void k_b_sp2_bounds(int n, const int *__restrict__ slots, const MolDe
   c.sp2_apply = 0;
 }
 
-// Per molecule (one 1,024-thread CTA): kLzSteps Lanczos steps on its extrapolated Fock
-// (d.X, before the SP2 map), the vectors in shared memory (3 nao doubles), and the SP2
-// interval narrowed to [theta_min - 3% R, theta_max + 5% R] inside the Gershgorin one that
-// k_b_sp2_bounds left in sp2_emin / sp2_emax (widened like it). Orders below 2 kLzSteps or
-// above kLzMaxOrder keep the Gershgorin interval. Deterministic: fixed-order reductions.
+// Per molecule: kLzSteps Lanczos steps on its extrapolated Fock (d.X, before the SP2 map), the
+// vectors in shared memory (3 nao doubles), and the SP2 interval narrowed to [theta_min - 3% R,
+// theta_max + 5% R] inside the Gershgorin one that k_b_sp2_bounds left in sp2_emin / sp2_emax
+// (widened like it). Orders below 2 kLzSteps or above kLzMaxOrder keep the Gershgorin interval.
+// One 1,024-thread CTA per molecule up to kLzOneCta orbitals, a cluster of kLzCluster above: one SM
+// reads a matrix at ~100 GB/s, so 16 passes over the 12 MB of 1,226 orbitals took 1.8 ms of each SCF
+// cycle with the GPU idle beside it (now 0.4); the CTAs share the rows of the mat-vec, hand each other
+// the results through distributed shared memory and run the recurrence themselves. Deterministic:
+// fixed-order reductions, the same for both forms.
 constexpr int kLzMaxOrder = 4096;
 __device__ __forceinline__ double lz_block_sum(double v, double *red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -558,15 +565,39 @@ __device__ int lz_sturm(const double *a, const double *b, int m, double x) {
   }
   return c;
 }
+// The smallest x with at least `target` eigenvalues of the Lanczos tridiagonal below it (one warp):
+// 32-point multisection, then bisection to neighbouring doubles. The count is monotonic in x, so
+// this is the x that bisection alone ends at; 200 dependent counts of 16 divisions by one thread took
+// 0.4 ms.
+__device__ double lz_end(const double *a, const double *b, double lo, double hi, int target, int lane) {
+  for (int round = 0; round < 9; ++round) {  // 33^9 = 4.6e13: some 100 ulps left
+    const double x = lo + (hi - lo) * ((double)(lane + 1) * (1.0 / 33.0));
+    const unsigned hit = __ballot_sync(0xffffffffu, lz_sturm(a, b, kLzSteps, x) >= target);
+    const int f = hit ? __ffs(hit) - 1 : 32;
+    const double xl = __shfl_sync(0xffffffffu, x, f > 0 ? f - 1 : 0), xh = __shfl_sync(0xffffffffu, x, f < 32 ? f : 31);
+    if (f > 0) lo = xl;
+    if (f < 32) hi = xh;
+  }
+  for (int it = 0; it < 100; ++it) {
+    const double mid = 0.5 * (lo + hi);
+    if (!(mid > lo && mid < hi)) break;
+    if (lz_sturm(a, b, kLzSteps, mid) >= target) hi = mid;
+    else lo = mid;
+  }
+  return hi;
+}
+
+constexpr int kLzOneCta = 320, kLzCluster = 8;
+template <int CN>
 __global__ void __launch_bounds__(1024) k_b_lanczos(BatchList L, const MolDesc *__restrict__ D,
                                                     MolCtl *__restrict__ C) {
   extern __shared__ double lzs[];
-  const int m = blockIdx.x;
+  const int m = blockIdx.x / CN, rank = blockIdx.x % CN;
   const int slot = L.slot[m];
   const MolDesc &d = D[slot];
   MolCtl &c = C[slot];
   const int n = d.g.nao;
-  if (n < 2 * kLzSteps || n > kLzMaxOrder) return;
+  if (n < 2 * kLzSteps || n > kLzMaxOrder || (n <= kLzOneCta) != (CN == 1)) return;  // (the whole cluster)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double *vp = lzs, *v = lzs + n, *w = lzs + 2 * n, *red = lzs + 3 * n;
   __shared__ double alpha[kLzSteps], beta[kLzSteps + 1];
@@ -583,7 +614,8 @@ __global__ void __launch_bounds__(1024) k_b_lanczos(BatchList L, const MolDesc *
   double bj = 0.0;
   for (int j = 0; j < kLzSteps; ++j) {
     __syncthreads();
-    for (int i = warp; i < n; i += 32) {  // w = X v, a warp per row
+    if (CN > 1) cg::this_cluster().sync();  // every CTA is done with the previous w
+    for (int i = rank * 32 + warp; i < n; i += 32 * CN) {  // w = X v, a warp per row
       const double *xi = d.X + (size_t)i * n;
       double acc = 0.0;
       for (int base = lane; base < n; base += 256) {
@@ -597,9 +629,14 @@ __global__ void __launch_bounds__(1024) k_b_lanczos(BatchList L, const MolDesc *
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) w[i] = acc;
+      if (CN == 1) {
+        if (lane == 0) w[i] = acc;
+      } else if (lane < CN) {
+        cg::this_cluster().map_shared_rank(w, lane)[i] = acc;
+      }
     }
-    __syncthreads();
+    if (CN > 1) cg::this_cluster().sync();
+    else __syncthreads();
     double a = 0.0;
     for (int i = threadIdx.x; i < n; i += 1024) a += w[i] * v[i];
     a = lz_block_sum(a, red);
@@ -623,28 +660,19 @@ __global__ void __launch_bounds__(1024) k_b_lanczos(BatchList L, const MolDesc *
     bj = b;
   }
   __syncthreads();
-  if (threadIdx.x != 0) return;
+  if (CN > 1) cg::this_cluster().sync();  // no CTA leaves while another may still write to it
+  if (rank != 0 || warp > 1) return;
   double g_lo = 1.0e300, g_hi = -1.0e300;
   for (int i = 0; i < kLzSteps; ++i) {
     const double r = (i > 0 ? fabs(beta[i]) : 0.0) + (i + 1 < kLzSteps ? fabs(beta[i + 1]) : 0.0);
     g_lo = fmin(g_lo, alpha[i] - r);
     g_hi = fmax(g_hi, alpha[i] + r);
   }
-  double lo = g_lo, hi = g_hi;
-  for (int it = 0; it < 100; ++it) {
-    const double mid = 0.5 * (lo + hi);
-    if (lz_sturm(alpha, beta, kLzSteps, mid) >= 1) hi = mid;
-    else lo = mid;
-  }
-  const double tmin = hi;
-  lo = g_lo;
-  hi = g_hi;
-  for (int it = 0; it < 100; ++it) {
-    const double mid = 0.5 * (lo + hi);
-    if (lz_sturm(alpha, beta, kLzSteps, mid) >= kLzSteps) hi = mid;
-    else lo = mid;
-  }
-  const double tmax = hi, R = tmax - tmin;
+  const double end = lz_end(alpha, beta, g_lo, g_hi, warp == 0 ? 1 : kLzSteps, lane);
+  if (lane == 0) red[warp] = end;
+  asm volatile("bar.sync 1, 64;" ::: "memory");  // the two warps
+  if (threadIdx.x != 0) return;
+  const double tmin = red[0], tmax = red[1], R = tmax - tmin;
   if (!(R > 0.0) || !isfinite(R)) return;
   const double elo = fmax(tmin - 0.03 * R, c.sp2_emin), ehi = fmin(tmax + 0.05 * R, c.sp2_emax);
   const double pad = 1.0e-3 * (ehi - elo) + 1.0e-6;
@@ -1314,6 +1342,9 @@ class BatchRunner {
     CUDA_OK(cudaStreamSynchronize(st_));
     CUDA_OK(cudaGetLastError());
     for (BatchMol *b : in) active_.push_back(b);
+    // largest first: their tiles run longest, so a grouped launch ends on short ones
+    std::stable_sort(active_.begin(), active_.end(),
+                     [](const BatchMol *a, const BatchMol *b) { return a->L.nao > b->L.nao; });
   }
 
   // One SCF iteration of every active molecule. Returns the molecules that finished
@@ -1782,12 +1813,29 @@ class BatchRunner {
     int nmax = 0;
     for (const BatchMol *b : mols) nmax = std::max(nmax, std::min(b->L.nao, kLzMaxOrder));
     if (nmax < 2 * kLzSteps) return;
-    const size_t smem = sizeof(double) * (3 * (size_t)nmax + 33);
-    if (smem > lz_smem_) {
-      CUDA_OK(cudaFuncSetAttribute(k_b_lanczos, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      lz_smem_ = smem;
+    if (nmax > kLzOneCta) {
+      const size_t smem = sizeof(double) * (3 * (size_t)nmax + 33);
+      if (smem > lz_smem_) {
+        CUDA_OK(cudaFuncSetAttribute(k_b_lanczos<kLzCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        lz_smem_ = smem;
+      }
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(L.mol.n * kLzCluster);
+      cfg.blockDim = dim3(1024);
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = st_;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = kLzCluster;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      CUDA_OK(cudaLaunchKernelEx(&cfg, k_b_lanczos<kLzCluster>, L.mol, (const MolDesc *)desc_, ctl_));
+      note_launch();
     }
-    k_b_lanczos<<<L.mol.n, 1024, smem, st_>>>(L.mol, desc_, ctl_);
+    k_b_lanczos<1><<<L.mol.n, 1024, sizeof(double) * (3 * (size_t)std::min(nmax, kLzOneCta) + 33), st_>>>(L.mol, desc_,
+                                                                                                          ctl_);
     note_launch();
   }
 
@@ -2067,7 +2115,7 @@ class BatchRunner {
   cudaEvent_t eig_done_ = nullptr;
   unsigned rside_ = 0;                // round robin over the side streams
   int side_used_ = 0;       // side streams with queued eigensolves not yet joined
-  size_t lz_smem_ = 48 * 1024;  // dynamic shared memory k_b_lanczos is set up for
+  size_t lz_smem_ = 48 * 1024;  // dynamic shared memory the clustered k_b_lanczos is set up for
   // Eigenvalues alone at retirement: the cluster kernel for every order it takes (it runs
   // asynchronously beside the next SCF step; cuSOLVER's dsyevd held the host thread for the
   // whole solve of each large molecule, ~1 s per 600 requests of the served stream).
