@@ -451,28 +451,60 @@ __device__ __forceinline__ int lorb(int i) { return i == 1 ? 0 : (i <= 4 ? 1 : 2
 
 // ---- one pair, one warp ------------------------------------------------------------
 
-constexpr int kVStride = 46;
-struct DPairShared {
+// Shared memory of one pair, for at most IJ x KL pair products (IJ those of the heavier atom). A
+// warp's latency is what a pair costs (three lanes work out the multipoles one after the other), so
+// what counts is how many warps an SM holds, and the largest pair (45 x 45, 34 KB) let it hold six.
+// Most pairs have no d atom (10 x 10, 3 KB) or one (45 x 10, 9 KB), so each kernel runs once per
+// class of pairs and skips the pairs of the others. A pair of two d atoms, 2,025 integrals, takes a
+// warp 1.3 ms; in the gradient it gets a block of T threads (as does one with one d atom), which
+// share out the work of a warp's lanes: 64 mixed chains of up to 60 atoms 114 -> 44 ms, a 41-atom
+// chain 3.0 -> 1.23 ms. The build keeps one warp a pair (the same chains 16.8 -> 5.0 and 2.1 -> 0.7 ms,
+// the overlaps' tables below included).
+enum DClass { kTwoD, kOneD, kNoD, kWithD };
+template <int IJ, int KL, int T, int C>
+struct DPairSharedT {
+  static constexpr int kClass = C;
+  static constexpr int kThreads = T, kVStride = KL + 1, kRep = IJ > 10 ? 492 : 35;
   RotPD R;
   double ri[23];
   double core[11][3];
-  double v[46 * kVStride];  // v[ij][kl], ij = indexd 1..45, kl = 1..limkl
-  double ww[2026];          // rep(1..491) during the first rotation, then ww(1..limij*limkl)
+  double v[(IJ + 1) * kVStride];  // v[ij][kl], ij = 1..limij, kl = 1..limkl
+  // rep(1 .. kRep - 1) during the first rotation, then ww(1..limij*limkl)
+  double ww[IJ * KL + 1 > kRep ? IJ * KL + 1 : kRep];
 };
+using DPairTwoD = DPairSharedT<45, 45, 512, kTwoD>;
+using DPairOneD = DPairSharedT<45, 10, 128, kOneD>;
+using DPairNoD = DPairSharedT<10, 10, 32, kNoD>;
+using DPairShared = DPairSharedT<45, 45, 32, kWithD>;  // any pair with a d atom, by one warp
+template <class S>
+__device__ __forceinline__ void pair_sync() {
+  if (S::kThreads == 32) __syncwarp();
+  else __syncthreads();
+}
+// Whether a pair of atoms with na and nb orbitals is one of class S's.
+template <class S>
+__device__ __forceinline__ bool pair_class(int na, int nb) {
+  const int hi = max(na, nb), lo = min(na, nb);
+  if (S::kClass == kTwoD) return lo == 9;
+  if (S::kClass == kOneD) return hi == 9 && lo < 9;
+  return S::kClass == kNoD ? hi < 9 : hi == 9;
+}
 
 // Computes the pair's molecular-frame w (left in S.ww, 1-based, row-major limij x limkl)
 // and the electron-core terms (S.core) for the ordered pair (ea, eb), displacement d = R_b - R_a.
-__device__ void warp_pair_d(DPairShared &S, const DTables *T, const ElementRec &ea, const ElementRec &eb, double dx,
+template <class Shared>
+__device__ void warp_pair_d(Shared &S, const DTables *tab, const ElementRec &ea, const ElementRec &eb, double dx,
                             double dy, double dz, int lane) {
+  constexpr int T = Shared::kThreads, kApart = T >= 128 ? 32 : 1;  // the three serial parts on warps of their own
   const bool has_d = ea.n_orb == 9 || eb.n_orb == 9;
   const double r = sqrt((dx * dx + dy * dy) + dz * dz);
   if (lane == 0) rotmat(dx, dy, dz, has_d, S.R);
-  if (lane == 1) reppd(ea, eb, r, S.ri);
-  if (lane == 2) spcore(ea, eb, r, S.core);
+  if (lane == kApart) reppd(ea, eb, r, S.ri);
+  if (lane == 2 * kApart) spcore(ea, eb, r, S.core);
   double *rep = S.ww;
-  for (int k = lane; k < 492; k += 32) rep[k] = 0.0;
-  __syncwarp();
-  for (int k = lane + 1; k <= 34; k += 32) rep[k] = S.ri[c_ipos[k]];
+  for (int k = lane; k < Shared::kRep; k += T) rep[k] = 0.0;
+  pair_sync<Shared>();
+  for (int k = lane + 1; k <= 34; k += T) rep[k] = S.ri[c_ipos[k]];
   double cf, pt;
   d_feather(r, cf, pt);
   if (has_d) {
@@ -481,43 +513,43 @@ __device__ void warp_pair_d(DPairShared &S, const DTables *T, const ElementRec &
     const int lasti = ea.n_orb == 9 ? 9 : (ea.n_orb == 1 ? 1 : 4);
     const int lastk = eb.n_orb == 9 ? 9 : (eb.n_orb == 1 ? 1 : 4);
     const int ni = lasti * (lasti + 1) / 2, nk = lastk * (lastk + 1) / 2;
-    for (int t = lane; t < ni * nk; t += 32) {
+    for (int t = lane; t < ni * nk; t += T) {
       const int qi = t / nk, qk = t - qi * nk;
       int i, j, k, l;
       pair_of(qi, i, j);
       pair_of(qk, k, l);
       const int ij = indexd(i, j), kl = indexd(k, l);
-      const int numb = T->ind2[(ij - 1) * 45 + (kl - 1)];
-      if (numb <= 34 || T->isym[numb] != 0) continue;
-      const double v = rijkl(T, ea, eb, ij, kl, lorb(i), lorb(j), lorb(k), lorb(l), 0, r) * kEv;
+      const int numb = tab->ind2[(ij - 1) * 45 + (kl - 1)];
+      if (numb <= 34 || tab->isym[numb] != 0) continue;
+      const double v = rijkl(tab, ea, eb, ij, kl, lorb(i), lorb(j), lorb(k), lorb(l), 0, r) * kEv;
       rep[numb] = (i == j && k == l) ? v * cf + padd : v * cf;
     }
     // the d electron-core terms core[5..10] (lanes 0-5: electrons of b, 6-11: of a)
     if (lane < 6 && eb.n_orb == 9) {
       const int kd[6] = {indexd(5, 1), indexd(5, 2), indexd(5, 5), indexd(6, 3), indexd(6, 6), indexd(8, 8)};
       const int l1[6] = {0, 1, 2, 1, 2, 2};
-      S.core[5 + lane][2] = -rijkl(T, ea, eb, 1, kd[lane], 0, 0, 2, l1[lane], 1, r) * (kEv * ea.core);
+      S.core[5 + lane][2] = -rijkl(tab, ea, eb, 1, kd[lane], 0, 0, 2, l1[lane], 1, r) * (kEv * ea.core);
     }
     if (lane >= 6 && lane < 12 && ea.n_orb == 9) {
       const int t = lane - 6;
       const int kd[6] = {indexd(5, 1), indexd(5, 2), indexd(5, 5), indexd(6, 3), indexd(6, 6), indexd(8, 8)};
       const int l1[6] = {0, 1, 2, 1, 2, 2};
-      S.core[5 + t][1] = -rijkl(T, ea, eb, kd[t], 1, 2, l1[t], 0, 0, 2, r) * (kEv * eb.core);
+      S.core[5 + t][1] = -rijkl(tab, ea, eb, kd[t], 1, 2, l1[t], 0, 0, 2, r) * (kEv * eb.core);
     }
-    __syncwarp();
-    for (int t = lane; t < ni * nk; t += 32) {
+    pair_sync<Shared>();
+    for (int t = lane; t < ni * nk; t += T) {
       const int qi = t / nk, qk = t - qi * nk;
       int i, j, k, l;
       pair_of(qi, i, j);
       pair_of(qk, k, l);
-      const int numb = T->ind2[(indexd(i, j) - 1) * 45 + (indexd(k, l) - 1)];
+      const int numb = tab->ind2[(indexd(i, j) - 1) * 45 + (indexd(k, l) - 1)];
       if (numb <= 34) continue;
-      const int nold = T->isym[numb];
+      const int nold = tab->isym[numb];
       if (nold >= 35) rep[numb] = rep[nold];
       else if (nold <= -35) rep[numb] = -rep[-nold];
     }
   }
-  __syncwarp();
+  pair_sync<Shared>();
   // Feather the electron-core terms toward the point charge (rotatd.F90:1160-1181):
   // all ten scale by cfrac, the charge-charge ones {1,3,4,7,9,10} add the point charge.
   if (lane < 10) {
@@ -535,15 +567,15 @@ __device__ void warp_pair_d(DPairShared &S, const DTables *T, const ElementRec &
   // First rotation (MOPAC tx): each lane owns rows ij of v.
   const int ii = ea.n_orb, kk = eb.n_orb;
   const int limij = ii * (ii + 1) / 2, limkl = kk * (kk + 1) / 2;
-  for (int q = lane; q < limij; q += 32) {
+  for (int q = lane; q < limij; q += T) {
     int i1, j1;
     pair_of(q, i1, j1);
     const int ij = indexd(i1, j1);
-    double *v = S.v + ij * kVStride;
+    double *v = S.v + (q + 1) * Shared::kVStride;
     for (int c = 0; c <= limkl; ++c) v[c] = 0.0;
     for (int k1 = 1; k1 <= kk; ++k1)
       for (int l1 = 1; l1 <= k1; ++l1) {
-        const int nd = T->ind2[(ij - 1) * 45 + (indexd(k1, l1) - 1)];
+        const int nd = tab->ind2[(ij - 1) * 45 + (indexd(k1, l1) - 1)];
         if (nd == 0) continue;
         const double w = rep[nd];
         switch (c_met[indx(k1, l1)]) {
@@ -594,15 +626,15 @@ __device__ void warp_pair_d(DPairShared &S, const DTables *T, const ElementRec &
         }
       }
   }
-  __syncwarp();
+  pair_sync<Shared>();
   // Second rotation (MOPAC rotatd): each lane owns columns kl of ww.
   double *ww = S.ww;
-  for (int kl = lane + 1; kl <= limkl; kl += 32) {
+  for (int kl = lane + 1; kl <= limkl; kl += T) {
     for (int p = 0; p < limij; ++p) ww[p * limkl + kl] = 0.0;
     auto at = [&](int i, int j) -> double & { return ww[(indx(i, j) - 1) * limkl + kl]; };
     for (int i1 = 1; i1 <= ii; ++i1)
       for (int j1 = 1; j1 <= i1; ++j1) {
-        const double w = S.v[indexd(i1, j1) * kVStride + kl];
+        const double w = S.v[indx(i1, j1) * Shared::kVStride + kl];
         switch (c_met[indx(i1, j1)]) {
           case 1: at(1, 1) = w; break;
           case 2:
@@ -625,13 +657,13 @@ __device__ void warp_pair_d(DPairShared &S, const DTables *T, const ElementRec &
             for (int i = 1; i <= 5; ++i) {
               at(i + 4, i + 4) += rot_dd(S.R, i, i1 - 4, j1 - 4) * w;
               for (int j = 1; j < i; ++j)
-                at(i + 4, j + 4) += rot_dd(S.R, T->inddd[(i - 1) * 5 + (j - 1)], i1 - 4, j1 - 4) * w;
+                at(i + 4, j + 4) += rot_dd(S.R, tab->inddd[(i - 1) * 5 + (j - 1)], i1 - 4, j1 - 4) * w;
             }
             break;
         }
       }
   }
-  __syncwarp();
+  pair_sync<Shared>();
   // PM7 d balance (mndod_twocenter.rs:919-1004): the mean of the two-centre d Coulomb
   // integrals is set to <ss|ss>. Small and sequential: lane 0.
   if (lane == 0 && (ea.iod > 0 || eb.iod > 0)) {
@@ -698,12 +730,13 @@ __device__ void warp_pair_d(DPairShared &S, const DTables *T, const ElementRec &
       core[10][2] += s;
     }
   }
-  __syncwarp();
+  pair_sync<Shared>();
 }
 
 // One element (i >= j, 1-based) of the electron-core block of atom n (1 = a, 2 = b),
 // MOPAC elenuc (mndod_twocenter.rs:1008-1047).
-__device__ double elenuc(const DPairShared &S, const DTables *T, int n, int i, int j) {
+template <class Shared>
+__device__ double elenuc(const Shared &S, const DTables *T, int n, int i, int j) {
   const int ind1 = i - 1, ind2 = j - 1;
   const double(*core)[3] = S.core;
   if (ind1 == 0) return core[1][n];
@@ -734,11 +767,31 @@ constexpr int kDWarps = kDPairsPerBlock;  // pairs (warps) per block
 
 // One near pair in the MNDO/d frame by one warp: w in (u, v) orientation and the packed
 // electron-core blocks of both atoms.
-__device__ __forceinline__ void near_d_pair(DPairShared &S, const DeviceParams &P, const int *__restrict__ z,
+// A block takes kDWarps items: a warp each, or one after the other with all threads.
+template <class Shared>
+constexpr int pair_block() {
+  return Shared::kThreads == 32 ? 32 * kDWarps : Shared::kThreads;
+}
+template <class Shared>
+constexpr size_t pair_smem() {
+  return sizeof(Shared) * (Shared::kThreads == 32 ? kDWarps : 1);
+}
+template <class Shared, class Fn>
+__device__ __forceinline__ void for_block_pairs(double *smem, Fn fn) {
+  Shared *S = reinterpret_cast<Shared *>(smem);
+  if (Shared::kThreads == 32)
+    fn(S[threadIdx.x >> 5], (int)(threadIdx.x >> 5), (int)(threadIdx.x & 31));
+  else
+    for (int k = 0; k < kDWarps; ++k) fn(*S, k, (int)threadIdx.x);
+}
+
+template <class Shared>
+__device__ __forceinline__ void near_d_pair(Shared &S, const DeviceParams &P, const int *__restrict__ z,
                                             const double *__restrict__ xyz, const NearPair q,
                                             double *__restrict__ w, double *__restrict__ ecore, int lane) {
   const ElementRec &eu = P.elements[z[q.u]];
   const ElementRec &ev = P.elements[z[q.v]];
+  if (!pair_class<Shared>(eu.n_orb, ev.n_orb)) return;
   const bool keep = eu.n_orb >= ev.n_orb;  // heavier-first ordering (hamiltonian.rs:388-392)
   const int a = keep ? q.u : q.v, b = keep ? q.v : q.u;
   const ElementRec &ea = keep ? eu : ev;
@@ -747,13 +800,13 @@ __device__ __forceinline__ void near_d_pair(DPairShared &S, const DeviceParams &
   warp_pair_d(S, P.tab, ea, eb, dx, dy, dz, lane);
   const int limij = ea.n_orb * (ea.n_orb + 1) / 2, limkl = eb.n_orb * (eb.n_orb + 1) / 2;
   double *wp = w + q.woff;
-  for (int t = lane; t < limij * limkl; t += 32) {
+  for (int t = lane; t < limij * limkl; t += Shared::kThreads) {
     const int pi = t / limkl, pj = t - pi * limkl;
     wp[keep ? t : pj * limij + pi] = S.ww[t + 1];
   }
   double *e_a = ecore + (keep ? q.eoff_u : q.eoff_v);
   double *e_b = ecore + (keep ? q.eoff_v : q.eoff_u);
-  for (int t = lane; t < limij + limkl; t += 32) {
+  for (int t = lane; t < limij + limkl; t += Shared::kThreads) {
     int mu, nu;
     if (t < limij) {
       unpack(t, mu, nu);
@@ -763,23 +816,25 @@ __device__ __forceinline__ void near_d_pair(DPairShared &S, const DeviceParams &
       e_b[t - limij] = elenuc(S, P.tab, 2, mu + 1, nu + 1);
     }
   }
-  __syncwarp();
+  pair_sync<Shared>();
 }
 
-// Near pairs in the MNDO/d frame, one warp per pair.
-__global__ void __launch_bounds__(32 * kDWarps) k_near_integrals_d(int n_near, const int *__restrict__ z,
+// Near pairs in the MNDO/d frame, one warp per pair of the class.
+template <class Shared>
+__global__ void __launch_bounds__(pair_block<Shared>()) k_near_integrals_d(int n_near, const int *__restrict__ z,
                                                                    const double *__restrict__ xyz,
                                                                    const NearPair *__restrict__ np, DeviceParams P,
                                                                    double *__restrict__ w, double *__restrict__ ecore) {
   extern __shared__ double smem_d[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int p = blockIdx.x * kDWarps + warp;
-  if (p >= n_near) return;
-  near_d_pair(reinterpret_cast<DPairShared *>(smem_d)[warp], P, z, xyz, np[p], w, ecore, lane);
+  for_block_pairs<Shared>(smem_d, [&](Shared &S, int k, int lane) {
+    const int p = blockIdx.x * kDWarps + k;
+    if (p < n_near) near_d_pair(S, P, z, xyz, np[p], w, ecore, lane);
+  });
 }
 
 // Batched: item = kDWarps consecutive near pairs of one molecule.
-__global__ void __launch_bounds__(32 * kDWarps) k_b_near_integrals_d(BatchList L, const MolDesc *__restrict__ D,
+template <class Shared>
+__global__ void __launch_bounds__(pair_block<Shared>()) k_b_near_integrals_d(BatchList L, const MolDesc *__restrict__ D,
                                                                      DeviceParams P) {
   extern __shared__ double smem_d[];
   const int item = blockIdx.x;
@@ -788,16 +843,38 @@ __global__ void __launch_bounds__(32 * kDWarps) k_b_near_integrals_d(BatchList L
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int p = (item - L.prefix[m]) * kDWarps + warp;
   if (p >= d.g.n_near) return;
-  near_d_pair(reinterpret_cast<DPairShared *>(smem_d)[warp], P, d.g.z, d.g.xyz, d.g.np[p], d.w, d.ecore, lane);
+  near_d_pair(reinterpret_cast<Shared *>(smem_d)[warp], P, d.g.z, d.g.xyz, d.g.np[p], d.w, d.ecore, lane);
 }
 
 // ---- general Slater overlaps (src/overlap_d.rs) -------------------------------------
 
-__device__ __forceinline__ double fact(int n) {
-  double f = 1.0;
-  for (int i = 1; i <= n; ++i) f = f * (double)i;
-  return f;
+// Binomials and factorials (exact), and the coefficients 2 / (m! (m + i + 1)) of bfn's series. Worked
+// out per term, with their divisions, they were nearly all of an overlap's time (0.7 ms a pair).
+__constant__ double c_binom[9][9] = {{1, 0, 0, 0, 0, 0, 0, 0, 0},
+                                  {1, 1, 0, 0, 0, 0, 0, 0, 0},
+                                  {1, 2, 1, 0, 0, 0, 0, 0, 0},
+                                  {1, 3, 3, 1, 0, 0, 0, 0, 0},
+                                  {1, 4, 6, 4, 1, 0, 0, 0, 0},
+                                  {1, 5, 10, 10, 5, 1, 0, 0, 0},
+                                  {1, 6, 15, 20, 15, 6, 1, 0, 0},
+                                  {1, 7, 21, 35, 35, 21, 7, 1, 0},
+                                  {1, 8, 28, 56, 70, 56, 28, 8, 1}};
+__constant__ double c_fact[13] = {1, 1, 2, 6, 24, 120, 720, 5040, 40320, 362880, 3628800, 39916800, 479001600};
+struct BfnTable {
+  double c[13][16];  // [i][m], 0 for odd m + i
+};
+constexpr BfnTable bfn_table() {
+  BfnTable t{};
+  for (int i = 0; i < 13; ++i) {
+    double f = 1.0;
+    for (int m = 0; m < 16; ++m) {
+      if (m != 0) f = f * (double)m;
+      t.c[i][m] = (double)(2 * ((m + i + 1) % 2)) / (f * (double)(m + i + 1));
+    }
+  }
+  return t;
 }
+__constant__ BfnTable c_bfn = bfn_table();
 
 // MOPAC bfn: B integrals bf[0..12] of x = (ua - ub) r / 2.
 __device__ void bfn(double x, double bf[13]) {
@@ -813,18 +890,17 @@ __device__ void bfn(double x, double bf[13]) {
     for (int i = 0; i <= 12; ++i) bf[i] = (double)(2 * ((i + 1) % 2)) / ((double)i + 1.0);
   } else {
     const int last = absx > 2.0 ? 15 : absx > 1.0 ? 12 : absx > 0.5 ? 7 : 6;
-    for (int i = 0; i <= 12; ++i) {
-      double y = 0.0, xf = 1.0, xm = 1.0;
-      for (int m = 0; m <= last; ++m) {
-        if (m != 0) {
-          xf = xf * (double)m;  // m!
-          xm = xm * (-x);       // (-x)^m
-        }
-        const double coeff = (double)(2 * ((m + i + 1) % 2)) / (xf * (double)(m + i + 1));
-        y = y + xm * coeff;
-      }
-      bf[i] = y;
+    double y[13];
+#pragma unroll
+    for (int i = 0; i <= 12; ++i) y[i] = 0.0;
+    double xm = 1.0;  // (-x)^m
+    for (int m = 0; m <= last; ++m) {
+      if (m != 0) xm = xm * (-x);
+#pragma unroll
+      for (int i = 0; i <= 12; ++i) y[i] = __fma_rn(xm, c_bfn.c[i][m], y[i]);
     }
+#pragma unroll
+    for (int i = 0; i <= 12; ++i) bf[i] = y[i];
   }
 }
 
@@ -836,11 +912,6 @@ __device__ __forceinline__ double aff(int la, int m, int i) {
     return 0.0;
   }
   return (la == 2 && m == 0 && i == 2) ? -0.5 : 0.0;
-}
-
-__device__ __forceinline__ double binom(int i, int j) {
-  if (j < 0 || j > i) return 0.0;
-  return fact(i) / (fact(j) * fact(i - j));
 }
 
 // MOPAC ss: Slater overlap of shells la1, lb1 (1 s, 2 p, 3 d), component m1 (1 sigma,
@@ -856,26 +927,30 @@ __device__ double ss(int na, int nb, int la1, int lb1, int m1, double ua, double
       const int ib = nb + j - lb, id = lb - j - m;
       double sum1 = 0.0;
       const int iab = ia + ib;
+      // (the coefficients are products of small integers: exact in any order)
       for (int k1 = 0; k1 <= ia; ++k1)
-        for (int k2 = 0; k2 <= ib; ++k2)
+        for (int k2 = 0; k2 <= ib; ++k2) {
+          const double c12 = c_binom[ia][k1] * c_binom[ib][k2];
           for (int k3 = 0; k3 <= ic; ++k3)
-            for (int k4 = 0; k4 <= id; ++k4)
+            for (int k4 = 0; k4 <= id; ++k4) {
+              const double c1234 = c12 * (c_binom[ic][k3] * c_binom[id][k4]);
               for (int k5 = 0; k5 <= m; ++k5) {
                 const int iaf = iab - k1 - k2 + k3 + k4 + 2 * k5;
                 for (int k6 = 0; k6 <= m; ++k6) {
                   const int ibf = k1 + k2 + k3 + k4 + 2 * k6;
                   const double sign = (double)(1 - 2 * ((m + k2 + k4 + k5 + k6) % 2));
-                  const double coeff =
-                      binom(id, k4) * binom(ic, k3) * binom(ib, k2) * binom(ia, k1) * binom(m, k5) * binom(m, k6) * sign;
-                  sum1 = sum1 + af[iaf] * bf[ibf] * coeff;
+                  const double coeff = c1234 * (c_binom[m][k5] * c_binom[m][k6] * sign);
+                  sum1 = __fma_rn(__dmul_rn(af[iaf], bf[ibf]), coeff, sum1);
                 }
               }
+            }
+        }
       sum = sum + sum1 * (aff(la, m, i) * aff(lb, m, j));
     }
   }
   double rpow = 1.0;
   for (int t = 0; t < na + nb + 1; ++t) rpow = rpow * r;
-  const double norm = sqrt(ua * ub / (fact(na + na) * fact(nb + nb)) * (double)((la + la + 1) * (lb + lb + 1)));
+  const double norm = sqrt(ua * ub / (c_fact[na + na] * c_fact[nb + nb]) * (double)((la + la + 1) * (lb + lb + 1)));
   return sum * rpow * (d_powi(ua, na) * d_powi(ub, nb) / 2.0 * norm);
 }
 
@@ -1134,42 +1209,53 @@ __global__ void k_grad_pairs_d(GradGeometry g, DeviceParams P) {
 // Near pair p and stencil point s, a warp per item: w and the electron-core blocks of the
 // warp-per-pair kernel at the displaced separation, contracted with the density (lanes over
 // elements, fixed xor tree), added to the pair's stencil energy.
-__global__ void __launch_bounds__(32 * kDWarps) k_grad_near_d(GradGeometry g, DeviceParams P) {
+template <class Shared>
+__global__ void __launch_bounds__(pair_block<Shared>()) k_grad_near_d(GradGeometry g, DeviceParams P) {
   extern __shared__ double smem_d[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long item = (long long)blockIdx.x * kDWarps + warp;
-  const int p = (int)(item / kStencil), s = (int)(item % kStencil);
-  if (p >= g.n_near) return;
-  DPairShared &S = reinterpret_cast<DPairShared *>(smem_d)[warp];
-  const NearPair np = g.np[p];
-  const int u = np.u < np.v ? np.u : np.v, v = np.u < np.v ? np.v : np.u;
-  const StencilPair q = stencil_pair(g, P, u, v, s);
-  const ElementRec &ea = P.elements[g.z[q.a]];
-  const ElementRec &eb = P.elements[g.z[q.b]];
-  warp_pair_d(S, P.tab, ea, eb, q.d[0], q.d[1], q.d[2], lane);
-  const int oa = g.aoff[q.a], ob = g.aoff[q.b];
-  const int limij = ea.n_orb * (ea.n_orb + 1) / 2, limkl = eb.n_orb * (eb.n_orb + 1) / 2;
-  double E = 0.0;
-  for (int t = lane; t < limij * limkl; t += 32) {
-    const int pi = t / limkl, pj = t - pi * limkl;
-    int mu, nu, la, si;
-    unpack(pi, mu, nu);
-    unpack(pj, la, si);
-    E += two_e_coef(g, oa, ob, mu, nu, la, si) * S.ww[t + 1];
-  }
-  for (int t = lane; t < limij + limkl; t += 32) {
-    int mu, nu;
-    if (t < limij) {
-      unpack(t, mu, nu);
-      E += ecore_coef(g, oa, mu, nu) * elenuc(S, P.tab, 1, mu + 1, nu + 1);
-    } else {
-      unpack(t - limij, mu, nu);
-      E += ecore_coef(g, ob, mu, nu) * elenuc(S, P.tab, 2, mu + 1, nu + 1);
+  for_block_pairs<Shared>(smem_d, [&](Shared &S, int k, int lane) {
+    constexpr int T = Shared::kThreads;
+    const long long item = (long long)blockIdx.x * kDWarps + k;
+    const int p = (int)(item / kStencil), s = (int)(item % kStencil);
+    if (p >= g.n_near) return;
+    const NearPair np = g.np[p];
+    const int u = np.u < np.v ? np.u : np.v, v = np.u < np.v ? np.v : np.u;
+    if (!pair_class<Shared>(P.elements[g.z[u]].n_orb, P.elements[g.z[v]].n_orb)) return;
+    const StencilPair q = stencil_pair(g, P, u, v, s);
+    const ElementRec &ea = P.elements[g.z[q.a]];
+    const ElementRec &eb = P.elements[g.z[q.b]];
+    warp_pair_d(S, P.tab, ea, eb, q.d[0], q.d[1], q.d[2], lane);
+    const int oa = g.aoff[q.a], ob = g.aoff[q.b];
+    const int limij = ea.n_orb * (ea.n_orb + 1) / 2, limkl = eb.n_orb * (eb.n_orb + 1) / 2;
+    // the coefficients by all threads (over the half-rotated integrals, which are done with), the sum
+    // by one warp's lanes
+    double *coef = S.v;
+    for (int t = lane; t < limij * limkl; t += T) {
+      const int pi = t / limkl, pj = t - pi * limkl;
+      int mu, nu, la, si;
+      unpack(pi, mu, nu);
+      unpack(pj, la, si);
+      coef[t] = two_e_coef(g, oa, ob, mu, nu, la, si);
     }
-  }
+    pair_sync<Shared>();
+    if (lane < 32) {
+      double E = 0.0;
+      for (int t = lane; t < limij * limkl; t += 32) E = __fma_rn(coef[t], S.ww[t + 1], E);
+      for (int t = lane; t < limij + limkl; t += 32) {
+        int mu, nu;
+        if (t < limij) {
+          unpack(t, mu, nu);
+          E += ecore_coef(g, oa, mu, nu) * elenuc(S, P.tab, 1, mu + 1, nu + 1);
+        } else {
+          unpack(t - limij, mu, nu);
+          E += ecore_coef(g, ob, mu, nu) * elenuc(S, P.tab, 2, mu + 1, nu + 1);
+        }
+      }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) E += __shfl_xor_sync(0xffffffffu, E, o);
-  if (lane == 0) g.E[tri_index(g.n_atoms, u, v) * kStencil + s] += E;
+      for (int o = 16; o > 0; o >>= 1) E += __shfl_xor_sync(0xffffffffu, E, o);
+      if (lane == 0) g.E[tri_index(g.n_atoms, u, v) * kStencil + s] += E;
+    }
+    pair_sync<Shared>();
+  });
 }
 
 // Sets a kernel's dynamic shared-memory limit once per (kernel, device).
@@ -1180,6 +1266,28 @@ void ensure_smem(const void *fn, size_t bytes) {
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lock(mu);
   if (done.insert({fn, dev}).second) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
+// One launch per class of pairs: of the gradient, of one molecule's build and of a batch's. The
+// builds keep to one warp a pair because a pair shared by a block compiles to other roundings of the
+// same sums (1e-16 of an integral), which may end an SCF an iteration sooner or later; one launch for
+// all pairs with a d atom is as fast in a molecule, where only the slowest pair counts.
+template <class Launch>
+void for_grad_classes(Launch launch) {
+  launch(DPairTwoD{});
+  launch(DPairOneD{});
+  launch(DPairNoD{});
+}
+template <class Launch>
+void for_build_classes(Launch launch) {
+  launch(DPairShared{});
+  launch(DPairNoD{});
+}
+template <class Launch>
+void for_batch_classes(Launch launch) {
+  launch(DPairSharedT<45, 45, 32, kTwoD>{});
+  launch(DPairSharedT<45, 10, 32, kOneD>{});
+  launch(DPairNoD{});
 }
 
 }  // namespace
@@ -1197,10 +1305,13 @@ void launch_pairs_all_d(cudaStream_t st, int n_atoms, const int *z, const double
 void launch_near_integrals_d(cudaStream_t st, int n_near, const int *z, const double *xyz, const NearPair *np,
                              const DeviceParams &P, double *w, double *ecore) {
   if (n_near == 0) return;
-  const size_t smem = sizeof(DPairShared) * kDWarps;
-  ensure_smem((const void *)k_near_integrals_d, smem);
-  k_near_integrals_d<<<(n_near + kDWarps - 1) / kDWarps, 32 * kDWarps, smem, st>>>(n_near, z, xyz, np, P, w, ecore);
-  note_launch();
+  for_build_classes([&](auto shared) {
+    using S = decltype(shared);
+    const size_t smem = pair_smem<S>();
+    ensure_smem((const void *)k_near_integrals_d<S>, smem);
+    k_near_integrals_d<S><<<(n_near + kDWarps - 1) / kDWarps, pair_block<S>(), smem, st>>>(n_near, z, xyz, np, P, w, ecore);
+    note_launch();
+  });
 }
 
 void launch_b_pairs_all_d(cudaStream_t st, const BatchList &L, const MolDesc *D, const DeviceParams &P) {
@@ -1211,10 +1322,13 @@ void launch_b_pairs_all_d(cudaStream_t st, const BatchList &L, const MolDesc *D,
 
 void launch_b_near_integrals_d(cudaStream_t st, const BatchList &L, const MolDesc *D, const DeviceParams &P) {
   if (L.total <= 0) return;
-  const size_t smem = sizeof(DPairShared) * kDWarps;
-  ensure_smem((const void *)k_b_near_integrals_d, smem);
-  k_b_near_integrals_d<<<L.total, 32 * kDWarps, smem, st>>>(L, D, P);
-  note_launch();
+  for_batch_classes([&](auto shared) {
+    using S = decltype(shared);
+    const size_t smem = pair_smem<S>();
+    ensure_smem((const void *)k_b_near_integrals_d<S>, smem);
+    k_b_near_integrals_d<S><<<L.total, pair_block<S>(), smem, st>>>(L, D, P);
+    note_launch();
+  });
 }
 
 void launch_grad_pairs_d(cudaStream_t st, const GradGeometry &g, const DeviceParams &P) {
@@ -1226,11 +1340,14 @@ void launch_grad_pairs_d(cudaStream_t st, const GradGeometry &g, const DevicePar
 
 void launch_grad_near_d(cudaStream_t st, const GradGeometry &g, const DeviceParams &P) {
   if (g.n_near <= 0) return;
-  const size_t smem = sizeof(DPairShared) * kDWarps;
-  ensure_smem((const void *)k_grad_near_d, smem);
   const size_t items = (size_t)g.n_near * kStencil;
-  k_grad_near_d<<<(unsigned)((items + kDWarps - 1) / kDWarps), 32 * kDWarps, smem, st>>>(g, P);
-  note_launch();
+  for_grad_classes([&](auto shared) {
+    using S = decltype(shared);
+    const size_t smem = pair_smem<S>();
+    ensure_smem((const void *)k_grad_near_d<S>, smem);
+    k_grad_near_d<S><<<(unsigned)((items + kDWarps - 1) / kDWarps), pair_block<S>(), smem, st>>>(g, P);
+    note_launch();
+  });
 }
 
 void launch_stage_pair_d(cudaStream_t st, const DeviceParams &P, int zi, int zj, const double d[3], double *w,
