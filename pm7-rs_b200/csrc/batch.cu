@@ -201,35 +201,33 @@ __global__ void __launch_bounds__(RB) k_b_dots_c(BatchList L, const MolDesc *__r
     for (int i = 0; i < 3 * kHist + 2; ++i) d.part[(size_t)r.q * kPart + 2 + i] = v[i];
 }
 
-// Per molecule: the chunk partials summed in chunk order: E_el of the iteration (for the
-// convergence test; the reported energy is the reference's fold, k_b_fold_energy), |E|^2
-// and the DIIS inner products.
-__global__ void k_b_reduce(int n, const int *__restrict__ slots, const MolDesc *__restrict__ D,
-                           MolCtl *__restrict__ C) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= n) return;
+// Per molecule, a warp: the chunk partials summed in chunk order, a lane per sum: E_el of the
+// iteration (for the convergence test; the reported energy is the reference's fold,
+// k_b_fold_energy), |E|^2 and the DIIS inner products.
+constexpr int kCtlWarps = 4;  // molecules per block of k_b_reduce and k_b_control
+static_assert(3 * kHist + 4 <= 32, "a lane per sum");
+__global__ void __launch_bounds__(32 * kCtlWarps) k_b_reduce(int n, const int *__restrict__ slots,
+                                                             const MolDesc *__restrict__ D, MolCtl *__restrict__ C) {
+  const int m = blockIdx.x * kCtlWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (m >= n || lane >= 3 * kHist + 4) return;
   const MolDesc &d = D[slots[m]];
   MolCtl &c = C[slots[m]];
-  const int nc = items_chunks(d.g.nao);
-  double e = 0.0;
-  for (int q = 0; q < nc; ++q) e += d.part[(size_t)q * kPart + 0];
-  c.e_elec = 0.5 * e;
-  double err2 = 0.0;
-  for (int q = 0; q < nc; ++q) err2 += d.part[(size_t)q * kPart + 1];
-  c.err2 = err2;
-  const int k = c.n_ord;
-  for (int t = 0; t < 3 * kHist + 2; ++t) {
-    const bool used = t < k || t == kHist || (t > kHist && t < kHist + 1 + k) || t == 2 * kHist + 1 ||
-                      (t >= 2 * kHist + 2 && t < 2 * kHist + 2 + k);
-    if (!used) continue;
-    double s = 0.0;
-    for (int q = 0; q < nc; ++q) s += d.part[(size_t)q * kPart + 2 + t];
-    if (t < kHist) c.ee[t] = s;
-    else if (t == kHist) c.ee[k] = s;
-    else if (t < 2 * kHist + 1) c.df_row[t - kHist - 1] = s;
-    else if (t == 2 * kHist + 1) c.df_row[k] = s;
-    else c.df_col[t - 2 * kHist - 2] = s;
-  }
+  const int nc = items_chunks(d.g.nao), k = c.n_ord;
+  const int t = lane - 2;  // the inner product (-2 the energy, -1 |E|^2)
+  const bool used = t < k || t == kHist || (t > kHist && t < kHist + 1 + k) || t == 2 * kHist + 1 ||
+                    (t >= 2 * kHist + 2 && t < 2 * kHist + 2 + k);
+  if (!used) return;
+  const double *part = d.part + lane;
+  double s = 0.0;
+#pragma unroll 8
+  for (int q = 0; q < nc; ++q) s += part[(size_t)q * kPart];
+  if (t == -2) c.e_elec = 0.5 * s;
+  else if (t == -1) c.err2 = s;
+  else if (t < kHist) c.ee[t] = s;
+  else if (t == kHist) c.ee[k] = s;
+  else if (t < 2 * kHist + 1) c.df_row[t - kHist - 1] = s;
+  else if (t == 2 * kHist + 1) c.df_row[k] = s;
+  else c.df_col[t - 2 * kHist - 2] = s;
 }
 
 // ---- the <= 9x9 extrapolation algebra (HistoryHost in scf_host.hpp) on the device ----
@@ -308,58 +306,72 @@ __device__ bool dev_cdiis(const MolCtl &c, double *w) {
   return false;
 }
 
-// Euclidean projection onto the probability simplex (sort-based).
-__device__ void simplex_project(const double *v, int n, double *out) {
-  double u[kHist];
-  for (int i = 0; i < n; ++i) u[i] = v[i];
-  for (int i = 1; i < n; ++i) {  // descending insertion sort
-    const double x = u[i];
-    int j = i - 1;
-    while (j >= 0 && u[j] < x) {
-      u[j + 1] = u[j];
-      --j;
-    }
-    u[j + 1] = x;
-  }
-  double css = 0.0, theta = 0.0;
-  for (int j = 0; j < n; ++j) {
-    css += u[j];
-    const double t = (css - 1.0) / (j + 1.0);
-    if (u[j] - t > 0.0) theta = t;
-  }
-  for (int i = 0; i < n; ++i) out[i] = fmax(v[i] - theta, 0.0);
-}
-
-// A-DIIS weights (scf.rs:1812-1916): projected gradient on the simplex.
-__device__ bool dev_adiis(const MolCtl &c, double *cw) {
-  const int n = c.n_ord;
+// A-DIIS weights (scf.rs:1812-1916): projected gradient on the simplex, by a warp, entry i of n on lane i
+// (weight in cw; `u` is the warp's row of kHist doubles). Up to 400 steps that depend on one another:
+// one thread took 8,000 clocks a step from arrays in local memory, and the molecules of a warp waited
+// for the slowest (1.7 ms a cycle of 512 molecules while any was in this phase). Every sum keeps the
+// order of the entries.
+__device__ bool warp_adiis(const MolCtl &c, int n, int lane, double *u, double &cw) {
   if (n < 2) return false;
-  const int last = n - 1;
-  double d[kHist], s[kHist * kHist], gr[kHist], trial[kHist], proj[kHist];
-  for (int i = 0; i < n; ++i) {
-    d[i] = x_at(c, i, last) - x_at(c, last, last);
-    for (int j = 0; j < n; ++j) s[i * n + j] = x_at(c, i, j) - x_at(c, i, last) - x_at(c, last, j) + x_at(c, last, last);
-  }
-  double l = 1.0e-12;
-  for (int i = 0; i < n; ++i) {
-    double row = 0.0;
-    for (int j = 0; j < n; ++j) row += fabs(s[i * n + j] + s[j * n + i]);
-    l = fmax(l, row);
-  }
-  const double lr = 1.0 / l;
-  for (int i = 0; i < n; ++i) cw[i] = 0.0;
-  cw[last] = 1.0;
-  for (int it = 0; it < 400; ++it) {
-    for (int k = 0; k < n; ++k) {
-      double acc = 2.0 * d[k];
-      for (int j = 0; j < n; ++j) acc += (s[k * n + j] + s[j * n + k]) * cw[j];
-      gr[k] = acc;
+  const int last = n - 1, i = min(lane, last);
+  const bool own = lane < n;
+  const double xll = x_at(c, last, last), xil = x_at(c, i, last), xli = x_at(c, last, i);
+  const double d2 = 2.0 * (xil - xll);
+  double t[kHist], row = 0.0;
+#pragma unroll
+  for (int j = 0; j < kHist; ++j) {
+    t[j] = 0.0;
+    if (j < n) {
+      const double sij = x_at(c, i, j) - xil - x_at(c, last, j) + xll;
+      const double sji = x_at(c, j, i) - x_at(c, j, last) - xli + xll;
+      t[j] = sij + sji;
+      row += fabs(t[j]);
     }
-    for (int i = 0; i < n; ++i) trial[i] = cw[i] - lr * gr[i];
-    simplex_project(trial, n, proj);
+  }
+  double l = fmax(1.0e-12, row);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) l = fmax(l, __shfl_xor_sync(0xffffffffu, l, o));
+  const double lr = 1.0 / l;
+  cw = lane == last ? 1.0 : 0.0;
+  for (int it = 0; it < 400; ++it) {
+    if (own) u[lane] = cw;
+    __syncwarp();
+    double acc = d2;
+#pragma unroll
+    for (int j = 0; j < kHist; ++j)
+      if (j < n) acc = __fma_rn(t[j], u[j], acc);
+    const double v = __fma_rn(-lr, acc, cw);
+    // Euclidean projection onto the probability simplex: the values in descending order, their running
+    // sums, and the last shift that leaves its value positive
+    int rank = 0;
+    for (int j = 0; j < n; ++j) {
+      const double w = __shfl_sync(0xffffffffu, v, j);
+      rank += w > v || (w == v && j < lane);
+    }
+    __syncwarp();
+    if (own) u[rank] = v;
+    __syncwarp();
+    double css = 0.0, mine = 0.0;
+#pragma unroll
+    for (int j = 0; j < kHist; ++j)
+      if (j < n) {
+        css += u[j];
+        if (j == lane) mine = css;
+      }
+    const double shift = (mine - 1.0) / (lane + 1.0);
+    const unsigned above = __ballot_sync(0xffffffffu, own && u[i] - shift > 0.0);
+    double theta = __shfl_sync(0xffffffffu, shift, above ? 31 - __clz(above) : 0);
+    if (!above) theta = 0.0;
+    const double proj = fmax(v - theta, 0.0);
+    __syncwarp();
+    if (own) u[lane] = fabs(proj - cw);
+    __syncwarp();
     double delta = 0.0;
-    for (int i = 0; i < n; ++i) delta += fabs(proj[i] - cw[i]);
-    for (int i = 0; i < n; ++i) cw[i] = proj[i];
+#pragma unroll
+    for (int j = 0; j < kHist; ++j)
+      if (j < n) delta += u[j];
+    cw = proj;
+    __syncwarp();
     if (delta < 1.0e-12) break;
   }
   return true;
@@ -370,43 +382,56 @@ __device__ bool dev_adiis(const MolCtl &c, double *cw) {
 constexpr double kMixedSwitch = 1.0e-3;
 constexpr double kMixedSwitchStep = 1.0e-6;  // rms density step that also ends the fp32 phase
 
-__global__ void k_b_control(int n, const int *__restrict__ slots, MolCtl *__restrict__ C,
-                            unsigned char *__restrict__ use32) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(32 * kCtlWarps) k_b_control(int n, const int *__restrict__ slots,
+                                                              MolCtl *C, unsigned char *use32) {
+  __shared__ double rows[kCtlWarps][kHist];
+  const int m = blockIdx.x * kCtlWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (m >= n) return;
   MolCtl &c = C[slots[m]];
-  // mixed precision: fp32 densities until the DIIS error is small, fp64 from then on
-  // (the first cycles' error says nothing: a SAD guess proportional to I commutes with F;
-  // for a large molecule the commutator norm can stall at the fp32 noise floor while the
-  // density step is already small, so either criterion, or 40 fp32 cycles, ends the phase)
-  if (c.mixed && c.iter >= 2 && (sqrt(c.err2) < kMixedSwitch || c.dp < kMixedSwitchStep || c.fp32_iters >= 40))
-    c.mixed = 0;
-  c.use32 = c.mixed;
-  use32[m] = (unsigned char)c.use32;
-  const int s = c.slot, k = c.n_ord;
-  for (int i = 0; i < k; ++i) {
-    const int o = c.ord[i];
-    c.gram[o * kHist + s] = c.gram[s * kHist + o] = c.ee[i];
-    c.xdf[s * kHist + o] = c.df_row[i];
-    c.xdf[o * kHist + s] = c.df_col[i];
+  // (C is not declared free of aliases: the lanes read what lane 0 writes here, and a compiler told
+  // that nothing else touches it may keep the values from before the barrier)
+  const int s = c.slot, k = __shfl_sync(0xffffffffu, c.n_ord, 0);
+  if (lane == 0) {
+    // mixed precision: fp32 densities until the DIIS error is small, fp64 from then on
+    // (the first cycles' error says nothing: a SAD guess proportional to I commutes with F;
+    // for a large molecule the commutator norm can stall at the fp32 noise floor while the
+    // density step is already small, so either criterion, or 40 fp32 cycles, ends the phase)
+    if (c.mixed && c.iter >= 2 && (sqrt(c.err2) < kMixedSwitch || c.dp < kMixedSwitchStep || c.fp32_iters >= 40))
+      c.mixed = 0;
+    c.use32 = c.mixed;
+    use32[m] = (unsigned char)c.use32;
+    for (int i = 0; i < k; ++i) {
+      const int o = c.ord[i];
+      c.gram[o * kHist + s] = c.gram[s * kHist + o] = c.ee[i];
+      c.xdf[s * kHist + o] = c.df_row[i];
+      c.xdf[o * kHist + s] = c.df_col[i];
+    }
+    c.gram[s * kHist + s] = c.ee[k];
+    c.xdf[s * kHist + s] = c.df_row[k];
+    c.ord[k] = s;
+    c.n_ord = k + 1;
   }
-  c.gram[s * kHist + s] = c.ee[k];
-  c.xdf[s * kHist + s] = c.df_row[k];
-  c.ord[k] = s;
-  c.n_ord = k + 1;
-  double w[kHist];
+  __syncwarp();
+  const bool cdiis = c.accel == 2 || sqrt(c.err2) <= c.adiis_switch;
+  double w[kHist], mine = 0.0;
   bool have = false;
   if (c.accel != 0) {
-    if (c.accel == 2 || sqrt(c.err2) <= c.adiis_switch) have = dev_cdiis(c, w);
-    else have = dev_adiis(c, w);
+    if (cdiis) {
+      if (lane == 0) have = dev_cdiis(c, w);
+    } else {
+      have = warp_adiis(c, k + 1, lane, rows[threadIdx.x >> 5], mine);
+#pragma unroll
+      for (int i = 0; i < kHist; ++i) w[i] = __shfl_sync(0xffffffffu, mine, i);
+    }
   }
+  if (lane != 0) return;
   if (!have) {
     c.ncoef = 1;
     c.csrc[0] = s;
     c.coef[0] = 1.0;
   } else {
     int q = 0;
-    for (int i = 0; i < c.n_ord; ++i)
+    for (int i = 0; i <= k; ++i)
       if (w[i] != 0.0) {  // an exact zero weight adds exactly nothing
         c.csrc[q] = c.ord[i];
         c.coef[q] = w[i];
@@ -1379,8 +1404,8 @@ class BatchRunner {
     {
       Stage s_(st_, "batch_diis");
       k_b_dots_c<<<A.chunks.total, RB, 0, st_>>>(A.chunks, desc_, ctl_);
-      k_b_reduce<<<nb, 128, 0, st_>>>(n, A.mol.slot, desc_, ctl_);
-      k_b_control<<<(n + 63) / 64, 64, 0, st_>>>(n, A.mol.slot, ctl_, flags_d_ + 2 * (size_t)cap_);
+      k_b_reduce<<<(n + kCtlWarps - 1) / kCtlWarps, 32 * kCtlWarps, 0, st_>>>(n, A.mol.slot, desc_, ctl_);
+      k_b_control<<<(n + kCtlWarps - 1) / kCtlWarps, 32 * kCtlWarps, 0, st_>>>(n, A.mol.slot, ctl_, flags_d_ + 2 * (size_t)cap_);
       note_launch(3);
     }
     // which molecules take an fp32 cycle (decided on the device from their DIIS error)
