@@ -408,7 +408,7 @@ struct DcSub {
 
 struct DcBucket {
   int np = 0, count = 0;  // matrices (2 per subsystem when unrestricted)
-  bool jacobi = false;    // solved by k_dc_jacobi (np <= kJacobiMax), else by cuSOLVER
+  bool jacobi = false;    // solved by k_jacobi (np <= kJacobiMax), else by cuSOLVER
   DevBuf<double> A, eps;
   DevBuf<int> info;
 };

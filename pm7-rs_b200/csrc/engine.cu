@@ -354,10 +354,9 @@ struct Eigen {
 // Eigendecomposition on the SCF path (`symmetric_eigen`, src/linalg.rs:231-278): cuSOLVER
 // dsyevd, or with PM7_DENSITY_SOLVER=jacobi the repo's Jacobi kernel for orders up to
 // kJacobiMax, warm-started from this object's previous eigenvectors (one object per spin
-// channel). Jacobi is not the default: measured per solve it is no faster than dsyevd at
-// ~60 orbitals and slower from ~100 (40 against 28 ms at 108), and on exactly degenerate
-// frontier levels (the reference's O2++ triplet and Cl- cases) its choice of vectors inside
-// the degenerate space leads the SCF to another state than the reference's. In place: A
+// channel). Jacobi is not the default: on exactly degenerate frontier levels (the
+// reference's O2++ triplet and Cl- cases) its choice of vectors inside the degenerate space
+// leads the SCF to another state than the reference's. In place: A
 // becomes the eigenvectors, one per row (row-major), eigenvalues ascending in eps(). A Jacobi
 // solve that ends unconverged or non-finite raises PM7_ERR_LINEAR_ALGEBRA at the next
 // check(), which the caller makes after a stream synchronisation.
