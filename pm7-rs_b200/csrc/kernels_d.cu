@@ -457,8 +457,8 @@ __device__ __forceinline__ int lorb(int i) { return i == 1 ? 0 : (i <= 4 ? 1 : 2
 // Most pairs have no d atom (10 x 10, 3 KB) or one (45 x 10, 9 KB), so each kernel runs once per
 // class of pairs and skips the pairs of the others. A pair of two d atoms, 2,025 integrals, takes a
 // warp 1.3 ms; in the gradient it gets a block of T threads (as does one with one d atom), which
-// share out the work of a warp's lanes: 64 mixed chains of up to 60 atoms 114 -> 44 ms, a 41-atom
-// chain 3.0 -> 1.23 ms. The build keeps one warp a pair (the same chains 16.8 -> 5.0 and 2.1 -> 0.7 ms,
+// share out the work of a warp's lanes: 64 molecules of 3 to 500 atoms 114 -> 44 ms, a chain of 41
+// heavy atoms 3.0 -> 1.23 ms. The build keeps one warp a pair (the same 16.8 -> 5.0 and 2.1 -> 0.7 ms,
 // the overlaps' tables below included).
 enum DClass { kTwoD, kOneD, kNoD, kWithD };
 template <int IJ, int KL, int T, int C>
