@@ -95,7 +95,7 @@ __device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
 // KC columns per thread; RR rows per CTA in registers (the last ones) and rs in shared memory (the
 // first), rs + RR <= 16. pub: 4 n doubles (two sets of p and next row).
 template <int KC, int RR>
-__global__ void __launch_bounds__(QT, 1) k_tridiag_grid(EigvalsTask T, int rs, double *__restrict__ pub,
+__global__ void __launch_bounds__(QT, 1) k_tridiag_grid(EigvalsTask T, int rs, double *pub,
                                                         unsigned *count, int *error) {
   extern __shared__ __align__(16) double tg_smem[];
   __shared__ double sums[2][QW], rows_red[2][QW][8], scal[4];
