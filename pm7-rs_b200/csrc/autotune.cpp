@@ -114,10 +114,24 @@ void save(const Store &s) {
 }  // namespace
 
 int autotune(cudaStream_t st, const std::string &key, int n_variants, const std::function<void(int)> &launch) {
-  if (n_variants <= 1) {
-    launch(0);
-    return 0;
-  }
+  int used = 0;
+  autotune_checked(
+      st, key, n_variants,
+      [&](int v) {
+        launch(v);
+        return cudaSuccess;
+      },
+      &used);
+  return used;
+}
+
+cudaError_t autotune_checked(cudaStream_t st, const std::string &key, int n_variants,
+                             const std::function<cudaError_t(int)> &launch, int *used) {
+  auto only = [&](int v) {
+    if (used) *used = v;
+    return launch(v);
+  };
+  if (n_variants <= 1) return only(0);
   Store &s = store();
   const std::string full = device_name() + "|" + key;
   {
@@ -126,42 +140,43 @@ int autotune(cudaStream_t st, const std::string &key, int n_variants, const std:
     for (const auto &f : s.forced)
       if (key.compare(0, f.first.size(), f.first) == 0 && f.second >= 0 && f.second < n_variants) {
         s.entries[full].choice = f.second;
-        launch(f.second);
-        return f.second;
+        return only(f.second);
       }
     auto it = s.entries.find(full);
     if (it != s.entries.end() && it->second.choice >= 0 && it->second.choice < n_variants) {
-      launch(it->second.choice);
-      return it->second.choice;
+      return only(it->second.choice);
     }
   }
   // one untimed run of every variant (first-launch costs), then one timed run each
   cudaEvent_t a, b;
-  if (cudaEventCreate(&a) != cudaSuccess || cudaEventCreate(&b) != cudaSuccess) {
-    launch(0);
-    return 0;
-  }
+  if (cudaEventCreate(&a) != cudaSuccess || cudaEventCreate(&b) != cudaSuccess) return only(0);
   std::vector<float> ms(n_variants, 0.0f);
-  for (int v = 0; v < n_variants; ++v) launch(v);
+  std::vector<cudaError_t> status(n_variants, cudaSuccess);
+  for (int v = 0; v < n_variants; ++v) status[v] = launch(v);
   for (int v = 0; v < n_variants; ++v) {
+    if (status[v] != cudaSuccess) continue;
     cudaEventRecord(a, st);
-    launch(v);
+    status[v] = launch(v);
     cudaEventRecord(b, st);
     cudaEventSynchronize(b);
     cudaEventElapsedTime(&ms[v], a, b);
   }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
-  int best = 0;
-  for (int v = 1; v < n_variants; ++v)
-    if (ms[v] < ms[best]) best = v;
+  int best = -1;
+  for (int v = 0; v < n_variants; ++v)
+    if (status[v] == cudaSuccess && (best < 0 || ms[v] < ms[best])) best = v;
+  if (best < 0) return status[0];
+  for (int v = 0; v < n_variants; ++v)
+    if (status[v] != cudaSuccess) ms[v] = -1.0f;  // (in the cache file: never ran)
   std::lock_guard<std::mutex> lock(s.mu);
   Entry e;
   e.choice = best;
   e.ms = ms;
   s.entries[full] = e;
   save(s);
-  return best;
+  if (used) *used = best;
+  return cudaSuccess;
 }
 
 std::string autotune_report() {

@@ -16,6 +16,12 @@ namespace pm7 {
 // for use inside a stream capture.
 int autotune(cudaStream_t st, const std::string &key, int n_variants, const std::function<void(int)> &launch);
 
+// The same for launches that can be refused (cooperative ones): launch(v) returns its status, which
+// this returns too. While timing, a variant whose launch fails is passed over and never kept; when all
+// fail nothing is kept and the first status is returned.
+cudaError_t autotune_checked(cudaStream_t st, const std::string &key, int n_variants,
+                             const std::function<cudaError_t(int)> &launch, int *used = nullptr);
+
 // The decisions so far as JSON ({"<device>|<key>": variant, ...}).
 std::string autotune_report();
 

@@ -586,8 +586,8 @@ struct Purifier {
     if (mode == 2) bounds_of(F, true);
     {
       Stage g_(st, "sp2_grid");
-      launch_sp2_purify(st, n, F, mode, (double)n_occ, w, rule, X.p, X2.p, P, grid_ws.p, bounds.p, state.p,
-                        grid_count.p, grid_err.p);
+      CUDA_OK(launch_sp2_purify(st, n, F, mode, (double)n_occ, w, rule, X.p, X2.p, P, grid_ws.p, bounds.p, state.p,
+                                grid_count.p, grid_err.p));
     }
     int *bad = reinterpret_cast<int *>(pin + kSp2Len);
     CUDA_OK(cudaMemcpyAsync(pin, state.p, kSp2Len * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -601,7 +601,7 @@ struct Purifier {
   void bounds_of(const double *F, bool refine) {
     if (n <= kSp2BoundsMax) {
       Stage l_(st, "sp2_bounds");
-      launch_sp2_bounds(st, n, F, refine, grid_ws.p, bounds.p, grid_count.p, grid_err.p);
+      CUDA_OK(launch_sp2_bounds(st, n, F, refine, grid_ws.p, bounds.p, grid_count.p, grid_err.p));
       return;
     }
     launch_gershgorin(st, n, F, scratch.p, bounds.p);

@@ -248,16 +248,17 @@ void launch_sp2_decide(cudaStream_t st, double n_occ, double *state, const doubl
 // A whole purification in one cooperative launch, and its spectral bounds alone
 // (kernels_sp2.cu). F is n x n; x0, x1 are sp2_grid_ld(n)^2; ws sp2_grid_doubles(n), zeroed once; P becomes
 // w times the projector; lanczos 1: narrowed bounds, 0: Gershgorin, 2: those in `bounds`. The
-// last step's Sp2State is left in state; count is a scratch counter; *error becomes 1 when a
-// grid barrier expired. launch_sp2_bounds takes n up to kSp2BoundsMax.
+// last step's Sp2State is left in state (kSp2Ok is 0 until then); count is a scratch counter; *error
+// becomes 1 when a grid barrier expired. Both return the launch's status: a cooperative grid can be
+// refused. launch_sp2_bounds takes n up to kSp2BoundsMax.
 constexpr int kSp2BoundsMax = 9400;  // three Lanczos vectors in one CTA's shared memory
 int sp2_grid_ld(int n);
 size_t sp2_grid_doubles(int n);
-void launch_sp2_bounds(cudaStream_t st, int n, const double *F, bool lanczos, double *ws, double *bounds,
-                       unsigned *count, int *error);
-void launch_sp2_purify(cudaStream_t st, int n, const double *F, int lanczos, double n_occ, double w, Sp2Rule rule,
-                       double *x0, double *x1, double *P, double *ws, double *bounds, double *state, unsigned *count,
-                       int *error);
+cudaError_t launch_sp2_bounds(cudaStream_t st, int n, const double *F, bool lanczos, double *ws, double *bounds,
+                              unsigned *count, int *error);
+cudaError_t launch_sp2_purify(cudaStream_t st, int n, const double *F, int lanczos, double n_occ, double w,
+                              Sp2Rule rule, double *x0, double *x1, double *P, double *ws, double *bounds,
+                              double *state, unsigned *count, int *error);
 }
 
 namespace pm7 {

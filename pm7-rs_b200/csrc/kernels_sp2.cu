@@ -727,11 +727,13 @@ int grid_sms() {
   return std::min(s, kMaxCtas);
 }
 
-void grid_launch(cudaStream_t st, const void *fn, int ctas, int threads, size_t smem, Sp2GridArgs &A) {
-  cudaMemsetAsync(A.count, 0, sizeof(unsigned), st);
+cudaError_t grid_launch(cudaStream_t st, const void *fn, int ctas, int threads, size_t smem, Sp2GridArgs &A) {
+  cudaError_t err = cudaMemsetAsync(A.count, 0, sizeof(unsigned), st);
   void *args[] = {&A};
-  cudaLaunchCooperativeKernel(fn, dim3(ctas), dim3(threads), args, smem, st);
+  if (err == cudaSuccess) err = cudaLaunchCooperativeKernel(fn, dim3(ctas), dim3(threads), args, smem, st);
   note_launch();
+  if (err != cudaSuccess) cudaGetLastError();  // the status is returned; no later check is to find it again
+  return err;
 }
 
 }  // namespace
@@ -739,8 +741,8 @@ void grid_launch(cudaStream_t st, const void *fn, int ctas, int threads, size_t 
 int sp2_grid_ld(int n) { return (n + TS - 1) / TS * TS; }
 size_t sp2_grid_doubles(int n) { return WsLayout(n).total; }
 
-void launch_sp2_bounds(cudaStream_t st, int n, const double *F, bool lanczos, double *ws, double *bounds,
-                       unsigned *count, int *error) {
+cudaError_t launch_sp2_bounds(cudaStream_t st, int n, const double *F, bool lanczos, double *ws, double *bounds,
+                              unsigned *count, int *error) {
   const int sms = grid_sms();
   Sp2GridArgs A{};
   A.n = n;
@@ -751,16 +753,16 @@ void launch_sp2_bounds(cudaStream_t st, int n, const double *F, bool lanczos, do
   A.count = count;
   A.error = error;
   const int rows = kBoundsThreads / 256;  // at a time per CTA
-  grid_launch(st, (const void *)k_sp2_bounds, std::min(sms, (n + rows - 1) / rows), kBoundsThreads,
-              3 * (size_t)n * 8, A);
+  return grid_launch(st, (const void *)k_sp2_bounds, std::min(sms, (n + rows - 1) / rows), kBoundsThreads,
+                     3 * (size_t)n * 8, A);
 }
 
 // The grid of a purification: a CTA per SM at most, no more than there are tiles or (so that a
 // CTA keeps its rows of F in registers through the Lanczos steps) row sets; or, the tuner's other
 // variant, the fewest CTAs that take the tiles in as many waves, whose barriers are cheaper.
-void launch_sp2_purify(cudaStream_t st, int n, const double *F, int lanczos, double n_occ, double w, Sp2Rule rule,
-                       double *x0, double *x1, double *P, double *ws, double *bounds, double *state, unsigned *count,
-                       int *error) {
+cudaError_t launch_sp2_purify(cudaStream_t st, int n, const double *F, int lanczos, double n_occ, double w,
+                              Sp2Rule rule, double *x0, double *x1, double *P, double *ws, double *bounds,
+                              double *state, unsigned *count, int *error) {
   const int sms = grid_sms();
   Sp2GridArgs A{};
   A.n = n;
@@ -779,7 +781,8 @@ void launch_sp2_purify(cudaStream_t st, int n, const double *F, int lanczos, dou
   A.count = count;
   A.error = error;
   if (lanczos == 1 && 3 * (size_t)n * 8 > kSmem) {  // the Lanczos vectors need the other kernel's shared memory
-    launch_sp2_bounds(st, n, F, true, ws, bounds, count, error);
+    const cudaError_t err = launch_sp2_bounds(st, n, F, true, ws, bounds, count, error);
+    if (err != cudaSuccess) return err;
     A.lanczos = 2;
   }
   const int tb = A.ld / TS, tiles = tb * (tb + 1) / 2, waves = (tiles + sms - 1) / sms;
@@ -787,8 +790,12 @@ void launch_sp2_purify(cudaStream_t st, int n, const double *F, int lanczos, dou
   const int most = std::min(sms, std::max(tiles, rows));
   const int even = std::min(sms, std::max((tiles + waves - 1) / waves, rows));
   const int bucket = ((n + 255) / 256) * 256;
-  autotune(st, "sp2_square|n" + std::to_string(bucket), 2,
-           [&](int v) { grid_launch(st, (const void *)k_sp2_purify, v == 0 ? most : even, GT, kSmem, A); });
+  // the verdict is "not settled" until a kernel that ran says otherwise
+  const cudaError_t err = cudaMemsetAsync(state + kSp2Ok, 0, sizeof(double), st);
+  if (err != cudaSuccess) return err;
+  return autotune_checked(st, "sp2_square|n" + std::to_string(bucket), 2, [&](int v) {
+    return grid_launch(st, (const void *)k_sp2_purify, v == 0 ? most : even, GT, kSmem, A);
+  });
 }
 
 }  // namespace pm7

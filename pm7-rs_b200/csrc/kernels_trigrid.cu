@@ -357,12 +357,13 @@ cudaError_t launch_tridiag_grid(cudaStream_t st, EigvalsTask t, int *error) {
   const GridShape g = grid_shape(t.n);
   double *pub = t.V;  // the blocked kernel's panel space
   unsigned *count = reinterpret_cast<unsigned *>(t.part + 4);
-  cudaMemsetAsync(count, 0, sizeof(unsigned), st);
+  cudaError_t err = cudaMemsetAsync(count, 0, sizeof(unsigned), st);
   int rs = g.rs;
   void *args[] = {&t, &rs, &pub, &count, &error};
-  const cudaError_t err = cudaLaunchCooperativeKernel(g.fn, dim3(g.ctas), dim3(QT), args,
-                                                      (size_t)(2 + rs) * t.n * 8, st);
+  if (err == cudaSuccess)
+    err = cudaLaunchCooperativeKernel(g.fn, dim3(g.ctas), dim3(QT), args, (size_t)(2 + rs) * t.n * 8, st);
   note_launch();
+  if (err != cudaSuccess) cudaGetLastError();  // the status is returned; no later check is to find it again
   return err;
 }
 
