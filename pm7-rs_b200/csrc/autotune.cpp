@@ -126,7 +126,7 @@ int autotune(cudaStream_t st, const std::string &key, int n_variants, const std:
 }
 
 cudaError_t autotune_checked(cudaStream_t st, const std::string &key, int n_variants,
-                             const std::function<cudaError_t(int)> &launch, int *used) {
+                             const std::function<cudaError_t(int)> &launch, int *used, bool alike) {
   auto only = [&](int v) {
     if (used) *used = v;
     return launch(v);
@@ -145,6 +145,10 @@ cudaError_t autotune_checked(cudaStream_t st, const std::string &key, int n_vari
     auto it = s.entries.find(full);
     if (it != s.entries.end() && it->second.choice >= 0 && it->second.choice < n_variants) {
       return only(it->second.choice);
+    }
+    if (alike) {
+      s.entries[full] = Entry{};
+      return only(0);
     }
   }
   // one untimed run of every variant (first-launch costs), then one timed run each

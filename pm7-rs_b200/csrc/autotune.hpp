@@ -18,9 +18,10 @@ int autotune(cudaStream_t st, const std::string &key, int n_variants, const std:
 
 // The same for launches that can be refused (cooperative ones): launch(v) returns its status, which
 // this returns too. While timing, a variant whose launch fails is passed over and never kept; when all
-// fail nothing is kept and the first status is returned.
+// fail nothing is kept and the first status is returned. alike: the variants of this key are one and
+// the same launch, so there is nothing to time: variant 0 is kept.
 cudaError_t autotune_checked(cudaStream_t st, const std::string &key, int n_variants,
-                             const std::function<cudaError_t(int)> &launch, int *used = nullptr);
+                             const std::function<cudaError_t(int)> &launch, int *used = nullptr, bool alike = false);
 
 // The decisions so far as JSON ({"<device>|<key>": variant, ...}).
 std::string autotune_report();

@@ -759,7 +759,9 @@ cudaError_t launch_sp2_bounds(cudaStream_t st, int n, const double *F, bool lanc
 
 // The grid of a purification: a CTA per SM at most, no more than there are tiles or (so that a
 // CTA keeps its rows of F in registers through the Lanczos steps) row sets; or, the tuner's other
-// variant, the fewest CTAs that take the tiles in as many waves, whose barriers are cheaper.
+// variant, the fewest CTAs that take the tiles in as many waves, whose barriers are cheaper. While one
+// wave takes all tiles the two are the same number and nothing is timed: a timing runs three extra
+// purifications (0.45 to 0.6 ms) in the first call of a size bucket.
 cudaError_t launch_sp2_purify(cudaStream_t st, int n, const double *F, int lanczos, double n_occ, double w,
                               Sp2Rule rule, double *x0, double *x1, double *P, double *ws, double *bounds,
                               double *state, unsigned *count, int *error) {
@@ -793,9 +795,11 @@ cudaError_t launch_sp2_purify(cudaStream_t st, int n, const double *F, int lancz
   // the verdict is "not settled" until a kernel that ran says otherwise
   const cudaError_t err = cudaMemsetAsync(state + kSp2Ok, 0, sizeof(double), st);
   if (err != cudaSuccess) return err;
-  return autotune_checked(st, "sp2_square|n" + std::to_string(bucket), 2, [&](int v) {
-    return grid_launch(st, (const void *)k_sp2_purify, v == 0 ? most : even, GT, kSmem, A);
-  });
+  auto launch = [&](int v) { return grid_launch(st, (const void *)k_sp2_purify, v == 0 ? most : even, GT, kSmem, A); };
+  const int bt = bucket / TS;
+  const bool alike = bt * (bt + 1) / 2 <= sms;  // one wave for every order of the bucket
+  if (!alike && most == even) return launch(0);
+  return autotune_checked(st, "sp2_square|n" + std::to_string(bucket), 2, launch, nullptr, alike);
 }
 
 }  // namespace pm7
