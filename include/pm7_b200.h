@@ -266,6 +266,13 @@ pm7_status pm7_stage_product_tf32(int32_t n, const double *a, const double *b, d
  * tr x_out and |x_out|_F^2 from the step's partials. A stage for accuracy tests. */
 pm7_status pm7_stage_sp2_step_i8(int32_t n, const double *x, int32_t square, double *x_out, double *norms);
 
+/* One SP2 purification as the SCF runs it: p_out (n x n) = 2 x the projector onto the n_occ lowest
+ * levels of the symmetric n x n matrix f. info (6 doubles) receives: 1 when it settled (p_out is
+ * meaningless otherwise), the Gershgorin retries, the steps, the spectral interval used, 1 when the
+ * integer tensor cores took the squarings. A stage for accuracy tests: the density half of
+ * `symmetric_eigen` + aufbau (src/linalg.rs:231-278, src/scf.rs:1148-1156) without the eigenvectors. */
+pm7_status pm7_stage_sp2(int32_t n, const double *f, int32_t n_occ, double *p_out, double info[6]);
+
 /* Failure drill of the bounded device waits (no counterpart in pm7-rs): runs the tcgen05
  * squaring of an n x n zero matrix (1 <= n <= 4096) with its copy producer withholding
  * every copy, so the pipeline's mbarrier waits never complete. Each wait gives up after its
@@ -305,6 +312,13 @@ pm7_status pm7_stage_corrections(const pm7_molecule *molecule, int32_t method,
 
 /* Number of CUDA kernels this library has launched since the process started. */
 int64_t pm7_launch_count(void);
+
+/* SP2 purifications since the process started, so that a density that quietly came from the
+ * eigensolver can be told from one that SP2 gave: out[0] asked for by single-molecule solves,
+ * out[1] of those repeated on the Gershgorin interval (the narrowed one had missed part of the
+ * spectrum), out[2] not settled (the solve diagonalised instead); out[3] asked for by batches,
+ * out[4] of those left to the batched eigensolver. */
+void pm7_sp2_counts(int64_t out[5]);
 
 /* The autotuner's decisions so far in this process, as JSON: {"<device>|<kernel key>":
  * variant, ...}. Result-identical launch variants (GEMM tile shapes, warps per block) are

@@ -1430,6 +1430,7 @@ class BatchRunner {
     }
     if (!purify64.empty() || !purify32.empty()) {
       Stage s_(st_, "batch_sp2");
+      note_sp2(kSp2BatchAsked, (int)(purify64.size() + purify32.size()));
       Lists S = lists(purify64, false, &up_sp2_);
       Lists T = lists(purify32, false, &up_sp32_);
       unsigned char *f64 = flags_d_, *f32 = flags_d_ + cap_;
@@ -1501,11 +1502,13 @@ class BatchRunner {
       for (int m = 0; m < S.mol.n; ++m)
         if (flags_h_[m] != 1) {
           fallback.push_back(purify64[m]);
+          note_sp2(kSp2BatchUnsettled);
           ++sp2_fallbacks_;
         }
       for (int m = 0; m < T.mol.n; ++m)
         if (flags_h_[cap_ + m] != 1) {
           fallback.push_back(purify32[m]);
+          note_sp2(kSp2BatchUnsettled);
           ++sp2_fallbacks_;
         }
       if (T.mol.n) {

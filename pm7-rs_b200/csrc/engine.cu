@@ -45,6 +45,8 @@ thread_local std::string g_last_error = "";
 // ---------------------------------------------------------------------------
 static std::atomic<long long> g_launches{0};
 void note_launch(int kernels) { g_launches.fetch_add(kernels, std::memory_order_relaxed); }
+static std::atomic<long long> g_sp2[kSp2Counts];
+void note_sp2(Sp2Count what, int by) { g_sp2[what].fetch_add(by, std::memory_order_relaxed); }
 
 StageProfiler g_prof;
 
@@ -525,6 +527,12 @@ struct Purifier {
   // fp32 iterate reaches idempotency only to its rounding floor, so the density carries
   // about 1e-5 relative error: the SCF uses it for its early cycles only.
   bool project32(const double *F, int n_occ, double w, double *P) {
+    note_sp2(kSp2Asked);
+    const bool ok = settle32(F, n_occ, w, P);
+    if (!ok) note_sp2(kSp2Unsettled);
+    return ok;
+  }
+  bool settle32(const double *F, int n_occ, double w, double *P) {
     ensure32();
     launch_gershgorin(st, n, F, scratch.p, bounds.p);
     launch_sp2_init32(st, n, ld, F, bounds.p, X32.p, hi32.p, lo32.p);
@@ -611,6 +619,12 @@ struct Purifier {
     launch_lanczos_bounds(st, n, F, lz.p, bounds.p);
   }
   bool project(const double *F, int n_occ, double w, double *P) {
+    note_sp2(kSp2Asked);
+    const bool ok = settle(F, n_occ, w, P);
+    if (!ok) note_sp2(kSp2Unsettled);
+    return ok;
+  }
+  bool settle(const double *F, int n_occ, double w, double *P) {
     ensure_grid();
     for (int attempt = 0; attempt < 2; ++attempt) {
       const bool refine = tight && attempt == 0;
@@ -619,6 +633,7 @@ struct Purifier {
       if (ok) return true;
       if (!refine) return false;
       tight = false;  // the refined interval missed part of the spectrum: Gershgorin from now on
+      note_sp2(kSp2Retried);
     }
     return false;
   }
@@ -2056,6 +2071,32 @@ pm7_status pm7_stage_sp2_step_i8(int32_t n, const double *x, int32_t square, dou
   });
 }
 
+pm7_status pm7_stage_sp2(int32_t n, const double *f, int32_t n_occ, double *p_out, double info[6]) {
+  return guarded([&] {
+    if (n < 1 || n_occ < 0 || n_occ > n || !f || !p_out || !info)
+      throw Failure{PM7_ERR_INVALID_INPUT, "stage_sp2 needs n >= 1, 0 <= n_occ <= n and buffers"};
+    DeviceContext &ctx = context_for(0);
+    std::lock_guard<std::mutex> lock(ctx.run_mutex);
+    CUDA_OK(cudaSetDevice(ctx.device));
+    cudaStream_t st = ctx.stream;
+    const size_t nn = (size_t)n * n;
+    DevBuf<double> F, P;
+    upload(F, std::vector<double>(f, f + nn), st);
+    P.alloc(nn, st);
+    Purifier pur(st, n, reinterpret_cast<double *>(ctx.pinned + 4096));
+    pur.i8 = use_i8_sp2(n);
+    const bool ok = pur.project(F.p, n_occ, 2.0, P.p);
+    CUDA_OK(cudaMemcpyAsync(p_out, P.p, sizeof(double) * nn, cudaMemcpyDeviceToHost, st));
+    CUDA_OK(cudaMemcpyAsync(info + 3, pur.bounds.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CUDA_OK(cudaStreamSynchronize(st));
+    CUDA_OK(cudaGetLastError());
+    info[0] = ok ? 1.0 : 0.0;
+    info[1] = pur.tight ? 0.0 : 1.0;
+    info[2] = pur.last_iterations;
+    info[5] = pur.i8 ? 1.0 : 0.0;
+  });
+}
+
 pm7_status pm7_stage_product_tf32(int32_t n, const double *a, const double *b, double *c_out) {
   return guarded([&] {
     if (n < 1 || !a || !b || !c_out) throw Failure{PM7_ERR_INVALID_INPUT, "product_tf32 needs n >= 1 and buffers"};
@@ -2190,6 +2231,10 @@ pm7_status pm7_stage_corrections(const pm7_molecule *molecule, int32_t method, i
 }
 
 int64_t pm7_launch_count(void) { return g_launches.load(); }
+
+void pm7_sp2_counts(int64_t out[5]) {
+  for (int k = 0; k < kSp2Counts; ++k) out[k] = g_sp2[k].load();
+}
 
 const char *pm7_autotune_report(void) {
   static thread_local std::string r;

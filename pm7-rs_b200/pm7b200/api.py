@@ -391,6 +391,14 @@ def launch_count():
     return int(lib().pm7_launch_count())
 
 
+def sp2_counts():
+    """SP2 purifications since process start and what became of them (`pm7_sp2_counts`)."""
+    out = (C.c_int64 * 5)()
+    lib().pm7_sp2_counts.restype = None
+    lib().pm7_sp2_counts(out)
+    return dict(zip(("asked", "retried", "unsettled", "batch_asked", "batch_unsettled"), (int(v) for v in out)))
+
+
 def profile_enable(on=True):
     lib().pm7_profile_enable.argtypes = [C.c_int32]
     lib().pm7_profile_enable(1 if on else 0)
@@ -620,6 +628,21 @@ def sp2_step_i8(x, square=True):
     _check(L.pm7_stage_sp2_step_i8(n, x.ctypes.data_as(abi.DP), int(bool(square)), out.ctypes.data_as(abi.DP),
                                    norms.ctypes.data_as(abi.DP)))
     return out, norms
+
+
+def sp2(f, n_occ):
+    """One SP2 purification (`pm7_stage_sp2`): (2 x the projector onto the n_occ lowest levels of f,
+    {settled, retries, steps, lo, hi, i8})."""
+    L = lib()
+    L.pm7_stage_sp2.argtypes = [C.c_int32, abi.DP, C.c_int32, abi.DP, abi.DP]
+    f = np.ascontiguousarray(f, dtype=np.float64)
+    n = f.shape[0]
+    out = np.zeros((n, n))
+    info = np.zeros(6)
+    _check(L.pm7_stage_sp2(n, f.ctypes.data_as(abi.DP), int(n_occ), out.ctypes.data_as(abi.DP),
+                           info.ctypes.data_as(abi.DP)))
+    return out, dict(settled=bool(info[0]), retries=int(info[1]), steps=int(info[2]), lo=info[3], hi=info[4],
+                     i8=bool(info[5]))
 
 
 def product_tf32(a, b):
