@@ -289,6 +289,12 @@ pm7_status pm7_stage_tf32_wait_drill(int32_t n);
 pm7_status pm7_stage_eigenvalues(int32_t count, const int32_t *orders, const double *a, double *w,
                                  int32_t device);
 
+/* Eigenvalues (ascending) of one symmetric matrix of order 2 .. 2048 through the whole-GPU
+ * reduction that gives the levels of a single-molecule solve, by `ctas` thread blocks (0: as many
+ * as the solve takes). The values do not depend on `ctas`, nor on the device's SM count. Fewer blocks
+ * than can hold the matrix are refused with PM7_ERR_INVALID_INPUT. A stage for accuracy tests. */
+pm7_status pm7_stage_levels(int32_t n, const double *a, int32_t ctas, double *w, int32_t device);
+
 /* Core-core repulsion energy in eV (`core_core_energy`, src/repulsion.rs:16-36). */
 pm7_status pm7_stage_core_core(const pm7_molecule *molecule, const pm7_params *params,
                                double *energy_ev);

@@ -2166,6 +2166,40 @@ pm7_status pm7_stage_eigenvalues(int32_t count, const int32_t *orders, const dou
   });
 }
 
+pm7_status pm7_stage_levels(int32_t n, const double *a, int32_t ctas, double *w, int32_t device) {
+  return guarded([&] {
+    DeviceContext &ctx = context_for(device);
+    std::lock_guard<std::mutex> lock(ctx.run_mutex);
+    CUDA_OK(cudaSetDevice(ctx.device));
+    if (!a || !w || !tridiag_grid_supported(n, ctas))
+      throw Failure{PM7_ERR_INVALID_INPUT, "levels: order " + std::to_string(n) + " on " + std::to_string(ctas) +
+                                               " blocks not supported, or null arrays"};
+    cudaStream_t st = ctx.stream;
+    const size_t nn = (size_t)n * n;
+    DevBuf<double> A, E, work;
+    DevBuf<EigvalsTask> task;
+    DevBuf<int> prefix, expired;
+    upload(A, std::vector<double>(a, a + nn), st);
+    E.alloc(n, st);
+    work.alloc(eigvals_work_doubles(n), st);
+    EigvalsTask t{};
+    t.src = A.p;
+    t.n = t.ld = n;
+    t.eps = E.p;
+    eigvals_task_layout(t, work.p);
+    upload(task, std::vector<EigvalsTask>{t}, st);
+    upload(prefix, std::vector<int>{0}, st);
+    upload(expired, std::vector<int>{0}, st);
+    CUDA_OK(launch_tridiag_grid(st, t, expired.p, ctas));
+    CUDA_OK(launch_tri_eigs(st, task.p, 1, prefix.p, n));
+    int e = 0;
+    CUDA_OK(cudaMemcpyAsync(&e, expired.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CUDA_OK(cudaMemcpyAsync(w, E.p, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
+    CUDA_OK(cudaStreamSynchronize(st));
+    if (e) throw Failure{PM7_ERR_TIMEOUT, "eigenvalue solve: a grid barrier expired"};
+  });
+}
+
 pm7_status pm7_stage_core_core(const pm7_molecule *molecule, const pm7_params *params, double *energy_ev) {
   return guarded([&] {
     Molecule m = to_molecule(molecule);

@@ -292,8 +292,9 @@ bool eigvals_supported(int n);
 // The reduction of one matrix by a cooperative launch over the whole GPU (kernels_trigrid.cu), in
 // place of k_tridiag; orders 2 .. kTriGridMax. *error becomes 1 when a grid barrier expired.
 constexpr int kTriGridMax = 2048;
-bool tridiag_grid_supported(int n);
-cudaError_t launch_tridiag_grid(cudaStream_t st, EigvalsTask t, int *error);
+// ctas: the grid's size (0: chosen by the order); the results are the same bits on every grid.
+bool tridiag_grid_supported(int n, int ctas = 0);
+cudaError_t launch_tridiag_grid(cudaStream_t st, EigvalsTask t, int *error, int ctas = 0);
 // The eigenvalues of already tridiagonal tasks (d, e^2, part): the second half of launch_eigvals.
 cudaError_t launch_tri_eigs(cudaStream_t st, const EigvalsTask *tasks, int n_tasks, const int *prefix, int total);
 // All tasks share one cluster size; prefix[t] = sum of the orders of tasks before t,

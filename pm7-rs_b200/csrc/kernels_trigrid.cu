@@ -4,14 +4,15 @@
 // exchanges between its owners; at n ~ 2,000 the products are 2/3 n^3 flop (0.2 ms of the chip's
 // FP64 rate), so the time is n times the latency of a column. The matrix is therefore kept on the
 // chip for the whole reduction: rows are dealt cyclically to the CTAs of a cooperative launch, and a
-// thread holds its columns (c = thread + 512 k) of up to 16 rows in registers, the rows that finish
-// first in shared memory. Nothing is blocked: the rank-2 update of a column is applied to the
+// thread holds its columns (c = thread + 512 k) of 4 rows (up to 512 columns) or 7 in registers, up to 8
+// more, the ones that finish first, in shared memory. Nothing is blocked: the rank-2 update of a column is applied to the
 // resident rows in the same pass that multiplies them with the next reflector, so a column needs ONE
 // grid barrier: each CTA publishes its rows' products p = A v and the owner of the next row that row,
 // not yet updated by the current reflector; after the barrier every CTA forms w, applies the update
 // to that row itself and derives the next reflector from it.
 //
-// Every sum is taken in a fixed order that depends on the matrix order alone.
+// Every sum is taken in a fixed order that depends on the matrix order alone, and a row's update is the
+// same chain of FMAs wherever the row lies, so the values are the same bits on every grid.
 //
 // Measured: 0.66 ms at 204 orbitals (cluster kernel 1.7), 0.87 at 270 (3.1), 2.4 at 666 and 10.9 at
 // 2,004 (cuSOLVER dsyevd, values included, 7.4 and 25.7): 3.2 to 5.4 us a column, of which the
@@ -93,7 +94,7 @@ __device__ __forceinline__ double warp_sum8(double (&v)[8], int lane) {
 }
 
 // KC columns per thread; RR rows per CTA in registers (the last ones) and rs in shared memory (the
-// first), rs + RR <= 16. pub: 4 n doubles (two sets of p and next row).
+// first), rs <= 8. pub: 4 n doubles (two sets of p and next row).
 template <int KC, int RR>
 __global__ void __launch_bounds__(QT, 1) k_tridiag_grid(EigvalsTask T, int rs, double *pub,
                                                         unsigned *count, int *error) {
@@ -186,9 +187,9 @@ __global__ void __launch_bounds__(QT, 1) k_tridiag_grid(EigvalsTask T, int rs, d
         for (int k = 0; k < KC; ++k) {
           const int c = tid + QT * k;
           if (c > j && c < n) {
-            const double y = row[c] - vi * wp[k] - wi * vp[k];
+            const double y = __fma_rn(-wi, vp[k], __fma_rn(-vi, wp[k], row[c]));
             row[c] = y;
-            acc += y * v[k];
+            acc = __fma_rn(y, v[k], acc);
             if (b == next_b && r == next_r) __stcg(grow + c, y);
           }
         }
@@ -203,8 +204,8 @@ __global__ void __launch_bounds__(QT, 1) k_tridiag_grid(EigvalsTask T, int rs, d
         double acc = 0.0;
 #pragma unroll
         for (int k = 0; k < KC; ++k) {
-          a[r][k] -= vi * wp[k] + wi * vp[k];
-          acc += a[r][k] * v[k];
+          a[r][k] = __fma_rn(-wi, vp[k], __fma_rn(-vi, wp[k], a[r][k]));
+          acc = __fma_rn(a[r][k], v[k], acc);
         }
         part[1][r] = acc;
         if (b == next_b && lr == next_r)
@@ -332,7 +333,7 @@ int tri_sms() {
 
 // Columns per thread by the order; as many CTAs as leave no more rows each than the registers hold,
 // at most one per SM, the rest of the rows in shared memory.
-GridShape grid_shape(int n) {
+GridShape grid_shape(int n, int ctas) {
   const int sms = tri_sms(), kc = (n + QT - 1) / QT;
   GridShape g{};
   g.rr = kc == 1 ? 4 : 7;
@@ -340,21 +341,21 @@ GridShape grid_shape(int n) {
          : kc == 2 ? (const void *)k_tridiag_grid<2, 7>
          : kc == 3 ? (const void *)k_tridiag_grid<3, 7>
                    : (const void *)k_tridiag_grid<4, 7>;
-  g.ctas = std::min(sms, (n + g.rr - 1) / g.rr);
+  g.ctas = ctas > 0 ? ctas : std::min(sms, (n + g.rr - 1) / g.rr);
   g.rs = std::max(0, (n + g.ctas - 1) / g.ctas - g.rr);
   return g;
 }
 
 }  // namespace
 
-bool tridiag_grid_supported(int n) {
-  if (n < 2 || n > kTriGridMax) return false;
-  const GridShape g = grid_shape(n);
+bool tridiag_grid_supported(int n, int ctas) {
+  if (n < 2 || n > kTriGridMax || ctas < 0 || ctas > std::min(n, tri_sms())) return false;
+  const GridShape g = grid_shape(n, ctas);
   return g.rs <= 8 && (size_t)(2 + g.rs) * n * 8 <= (size_t)kGridSmem;
 }
 
-cudaError_t launch_tridiag_grid(cudaStream_t st, EigvalsTask t, int *error) {
-  const GridShape g = grid_shape(t.n);
+cudaError_t launch_tridiag_grid(cudaStream_t st, EigvalsTask t, int *error, int ctas) {
+  const GridShape g = grid_shape(t.n, ctas);
   double *pub = t.V;  // the blocked kernel's panel space
   unsigned *count = reinterpret_cast<unsigned *>(t.part + 4);
   cudaError_t err = cudaMemsetAsync(count, 0, sizeof(unsigned), st);

@@ -616,6 +616,18 @@ def eigenvalues(matrices, device=0):
     return res
 
 
+def levels(a, ctas=0, device=0):
+    """Ascending eigenvalues of one symmetric matrix by the whole-GPU reduction
+    (`pm7_stage_levels`), on `ctas` thread blocks (0: the engine's own choice)."""
+    L = lib()
+    L.pm7_stage_levels.argtypes = [C.c_int32, abi.DP, C.c_int32, abi.DP, C.c_int32]
+    a = np.ascontiguousarray(a, dtype=np.float64)
+    out = np.zeros(a.shape[0])
+    _check(L.pm7_stage_levels(a.shape[0], a.ctypes.data_as(abi.DP), int(ctas), out.ctypes.data_as(abi.DP),
+                              int(device)))
+    return out
+
+
 def sp2_step_i8(x, square=True):
     """One fused FP64-accuracy SP2 step on the tcgen05 integer tensor cores (int8 digit
     planes): (x x or 2 x - x x, [tr, |.|_F^2] of it from the step's partials)."""
