@@ -256,6 +256,7 @@ void launch_sp2_decide(cudaStream_t st, double n_occ, double *state, const doubl
 // refused. launch_sp2_bounds takes n up to kSp2BoundsMax.
 constexpr int kSp2BoundsMax = 9400;  // three Lanczos vectors in one CTA's shared memory
 int sp2_grid_ld(int n);
+double sp2_sum_slack(int n);  // how far the purification's quick trace sums may be from the defining ones
 size_t sp2_grid_doubles(int n);
 cudaError_t launch_sp2_bounds(cudaStream_t st, int n, const double *F, bool lanczos, double *ws, double *bounds,
                               unsigned *count, int *error);

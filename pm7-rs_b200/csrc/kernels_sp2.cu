@@ -54,6 +54,7 @@ struct Sp2GridArgs {
   double *P;              // w * the projector, n x n
   double w, n_occ;
   Sp2Rule rule;
+  double slack;           // sp2_sum_slack(n)
   int lanczos;            // 1: Lanczos-narrowed bounds, 0: Gershgorin, 2: take bounds as given
   double *bounds;         // the interval used (in and out)
   double *state;          // Sp2State of the last step
@@ -605,12 +606,12 @@ __global__ void __launch_bounds__(GT) k_sp2_purify(Sp2GridArgs A) {
       // The iterate's traces tr X and tr X^2 = |X|_F^2, the branch (square when it brings the trace
       // closer to n_occ) and the stopping rule of sp2_control, the same in every CTA. The sums are
       // defined in one order (exact_traces), whose long chains of additions cost more than a small
-      // step; a quick sum differs from them by less than `off` (either order adds fewer than 100
-      // terms in a row), so it decides whenever no comparison is that close.
+      // step; a quick sum differs from them by less than `off` (A.slack: see sp2_sum_slack), so it
+      // decides whenever no comparison is that close.
       double trx, trx2;
       quick_traces(pin, norms, L, nb, n, step, at, lane, wpart, trx, trx2);
       double e = trx - trx2;
-      const double off = 1.0e-13 * (fabs(trx) + trx2) + 1.0e-15;
+      const double off = A.slack * (fabs(trx) + trx2) + 1.0e-15;
       const double d1 = fabs(trx2 - A.n_occ), d2 = fabs(2.0 * trx - trx2 - A.n_occ);
       if (!(fabs(e) > 1.0e-7 + 4.0 * off && fabs(d1 - d2) > 8.0 * off) || fabs(fabs(e) - A.rule.tol_floor) < 4.0 * off ||
           fabs(fabs(e) - A.rule.tol_done) < 4.0 * off || (step >= 2 && fabs(fabs(e) - fabs(ring[1])) < 8.0 * off)) {
@@ -738,6 +739,15 @@ cudaError_t grid_launch(cudaStream_t st, const void *fn, int ctas, int threads, 
 
 }  // namespace
 
+// What the quick sum and the defining sum of the same non-negative terms may differ by, relative to the
+// sum: a rounding (2^-53) per addition in the longest chain of each. Quick: 128 nb / 2,048 in a row, a tree
+// over 16, a warp, eight warps; defined: a row's two spans, 64 rows, nb / 256 blocks, a warp, eight
+// warps. 1e-13 covers 900 of them, up to 9,900 orbitals; beyond that the chains decide.
+double sp2_sum_slack(int n) {
+  const int nb = blocks64(n), quick = (128 * nb + 2047) / 2048 + 4 + 5 + 8, defined = 1 + 64 + (nb + 255) / 256 + 5 + 8;
+  return std::max(1.0e-13, (quick + defined + 1) * 1.1102230246251565e-16);
+}
+
 int sp2_grid_ld(int n) { return (n + TS - 1) / TS * TS; }
 size_t sp2_grid_doubles(int n) { return WsLayout(n).total; }
 
@@ -776,6 +786,7 @@ cudaError_t launch_sp2_purify(cudaStream_t st, int n, const double *F, int lancz
   A.w = w;
   A.n_occ = n_occ;
   A.rule = rule;
+  A.slack = sp2_sum_slack(n);
   A.lanczos = lanczos;
   A.bounds = bounds;
   A.state = state;
