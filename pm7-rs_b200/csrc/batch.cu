@@ -1164,6 +1164,8 @@ class BatchRunner {
     // kernel attributes of the SP2 steps, before any of them is captured into a graph
     prepare_gemm_kernels();
     prepare_tf32_kernels();
+    CUDA_OK(cudaFuncSetAttribute(k_b_lanczos<kLzCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)lz_smem(kLzMaxOrder)));
     CUDA_OK(cudaStreamCreateWithFlags(&eig_st_, cudaStreamNonBlocking));
     CUDA_OK(cudaEventCreateWithFlags(&eig_done_, cudaEventDisableTiming));
     for (Side &sd : side_) {
@@ -1836,17 +1838,16 @@ class BatchRunner {
     }
   }
 
-  // Lanczos-narrowed SP2 intervals for the molecules of list set L (vectors in shared memory).
+  static size_t lz_smem(int n) { return sizeof(double) * (3 * (size_t)n + 33); }
+  // Lanczos-narrowed SP2 intervals for the molecules of list set L (vectors in shared memory; the
+  // constructor has opted the clustered kernel in for the largest order: the limit belongs to the
+  // device, so a runner that set it for its own molecules took it from another that needs more).
   void launch_b_lanczos(const Lists &L, const std::vector<BatchMol *> &mols) {
     int nmax = 0;
     for (const BatchMol *b : mols) nmax = std::max(nmax, std::min(b->L.nao, kLzMaxOrder));
     if (nmax < 2 * kLzSteps) return;
     if (nmax > kLzOneCta) {
-      const size_t smem = sizeof(double) * (3 * (size_t)nmax + 33);
-      if (smem > lz_smem_) {
-        CUDA_OK(cudaFuncSetAttribute(k_b_lanczos<kLzCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        lz_smem_ = smem;
-      }
+      const size_t smem = lz_smem(nmax);
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(L.mol.n * kLzCluster);
       cfg.blockDim = dim3(1024);
@@ -1862,8 +1863,7 @@ class BatchRunner {
       CUDA_OK(cudaLaunchKernelEx(&cfg, k_b_lanczos<kLzCluster>, L.mol, (const MolDesc *)desc_, ctl_));
       note_launch();
     }
-    k_b_lanczos<1><<<L.mol.n, 1024, sizeof(double) * (3 * (size_t)std::min(nmax, kLzOneCta) + 33), st_>>>(L.mol, desc_,
-                                                                                                          ctl_);
+    k_b_lanczos<1><<<L.mol.n, 1024, lz_smem(std::min(nmax, kLzOneCta)), st_>>>(L.mol, desc_, ctl_);
     note_launch();
   }
 
@@ -2143,7 +2143,6 @@ class BatchRunner {
   cudaEvent_t eig_done_ = nullptr;
   unsigned rside_ = 0;                // round robin over the side streams
   int side_used_ = 0;       // side streams with queued eigensolves not yet joined
-  size_t lz_smem_ = 48 * 1024;  // dynamic shared memory the clustered k_b_lanczos is set up for
   // Eigenvalues alone at retirement: the cluster kernel for every order it takes (it runs
   // asynchronously beside the next SCF step; cuSOLVER's dsyevd held the host thread for the
   // whole solve of each large molecule, ~1 s per 600 requests of the served stream).
