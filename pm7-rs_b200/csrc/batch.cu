@@ -614,10 +614,10 @@ __device__ double lz_end(const double *a, const double *b, double lo, double hi,
 
 constexpr int kLzOneCta = 320, kLzCluster = 8;
 template <int CN>
-__global__ void __launch_bounds__(1024) k_b_lanczos(BatchList L, const MolDesc *__restrict__ D,
+__global__ void __launch_bounds__(1024) k_b_lanczos(BatchList L, int first, const MolDesc *__restrict__ D,
                                                     MolCtl *__restrict__ C) {
   extern __shared__ double lzs[];
-  const int m = blockIdx.x / CN, rank = blockIdx.x % CN;
+  const int m = first + blockIdx.x / CN, rank = blockIdx.x % CN;
   const int slot = L.slot[m];
   const MolDesc &d = D[slot];
   MolCtl &c = C[slot];
@@ -1842,14 +1842,21 @@ class BatchRunner {
   // Lanczos-narrowed SP2 intervals for the molecules of list set L (vectors in shared memory; the
   // constructor has opted the clustered kernel in for the largest order: the limit belongs to the
   // device, so a runner that set it for its own molecules took it from another that needs more).
+  // Each kernel gets its part of the list alone (sorted, largest first: see admit): eight empty CTAs of
+  // 1,024 threads for every small molecule cost a batch of 1,500 with one large one 0.05 ms of the 4.4
+  // that the densities of a cycle take.
   void launch_b_lanczos(const Lists &L, const std::vector<BatchMol *> &mols) {
-    int nmax = 0;
-    for (const BatchMol *b : mols) nmax = std::max(nmax, std::min(b->L.nao, kLzMaxOrder));
-    if (nmax < 2 * kLzSteps) return;
-    if (nmax > kLzOneCta) {
+    int nmax = 0, large = 0, used = 0;  // `large` first, then the others, up to `used`
+    for (int m = 0; m < (int)mols.size(); ++m) {
+      const int n = mols[m]->L.nao;
+      nmax = std::max(nmax, std::min(n, kLzMaxOrder));
+      if (n > kLzOneCta) large = m + 1;
+      if (n >= 2 * kLzSteps) used = m + 1;
+    }
+    if (large > 0) {
       const size_t smem = lz_smem(nmax);
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(L.mol.n * kLzCluster);
+      cfg.gridDim = dim3(large * kLzCluster);
       cfg.blockDim = dim3(1024);
       cfg.dynamicSmemBytes = smem;
       cfg.stream = st_;
@@ -1860,10 +1867,13 @@ class BatchRunner {
       at[0].val.clusterDim.z = 1;
       cfg.attrs = at;
       cfg.numAttrs = 1;
-      CUDA_OK(cudaLaunchKernelEx(&cfg, k_b_lanczos<kLzCluster>, L.mol, (const MolDesc *)desc_, ctl_));
+      CUDA_OK(cudaLaunchKernelEx(&cfg, k_b_lanczos<kLzCluster>, L.mol, 0, (const MolDesc *)desc_, ctl_));
       note_launch();
     }
-    k_b_lanczos<1><<<L.mol.n, 1024, lz_smem(std::min(nmax, kLzOneCta)), st_>>>(L.mol, desc_, ctl_);
+    int first = 0;  // what stands before it has all been taken above
+    while (first < large && mols[first]->L.nao > kLzOneCta) ++first;
+    if (first == used) return;
+    k_b_lanczos<1><<<used - first, 1024, lz_smem(std::min(nmax, kLzOneCta)), st_>>>(L.mol, first, desc_, ctl_);
     note_launch();
   }
 
