@@ -323,8 +323,8 @@ int64_t pm7_launch_count(void);
  * eigensolver can be told from one that SP2 gave: out[0] asked for by single-molecule solves,
  * out[1] of those repeated on the Gershgorin interval (the narrowed one had missed part of the
  * spectrum), out[2] not settled (the solve diagonalised instead); out[3] asked for by batches,
- * out[4] of those left to the batched eigensolver. */
-void pm7_sp2_counts(int64_t out[5]);
+ * out[4] of those left to the batched eigensolver; out[5] the squarings of out[0]. */
+void pm7_sp2_counts(int64_t out[6]);
 
 /* The autotuner's decisions so far in this process, as JSON: {"<device>|<kernel key>":
  * variant, ...}. Result-identical launch variants (GEMM tile shapes, warps per block) are

@@ -529,6 +529,7 @@ struct Purifier {
   bool project32(const double *F, int n_occ, double w, double *P) {
     note_sp2(kSp2Asked);
     const bool ok = settle32(F, n_occ, w, P);
+    note_sp2(kSp2Squarings, last_iterations);
     if (!ok) note_sp2(kSp2Unsettled);
     return ok;
   }
@@ -630,6 +631,7 @@ struct Purifier {
       const bool refine = tight && attempt == 0;
       const Sp2Rule rule{1.0e-13 * std::max(1, n_occ), 1.0e-6, kMaxSteps};
       const bool ok = i8 ? project_i8(F, n_occ, w, rule, refine, P) : project_grid(F, n_occ, w, rule, refine, P);
+      note_sp2(kSp2Squarings, last_iterations);
       if (ok) return true;
       if (!refine) return false;
       tight = false;  // the refined interval missed part of the spectrum: Gershgorin from now on
@@ -2266,7 +2268,7 @@ pm7_status pm7_stage_corrections(const pm7_molecule *molecule, int32_t method, i
 
 int64_t pm7_launch_count(void) { return g_launches.load(); }
 
-void pm7_sp2_counts(int64_t out[5]) {
+void pm7_sp2_counts(int64_t out[6]) {
   for (int k = 0; k < kSp2Counts; ++k) out[k] = g_sp2[k].load();
 }
 

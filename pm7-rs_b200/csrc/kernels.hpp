@@ -13,7 +13,7 @@ namespace pm7 {
 // Counts kernels launched by this library (read through pm7_launch_count()).
 void note_launch(int kernels = 1);
 // Counts SP2 purifications by what became of them (read through pm7_sp2_counts()).
-enum Sp2Count { kSp2Asked, kSp2Retried, kSp2Unsettled, kSp2BatchAsked, kSp2BatchUnsettled, kSp2Counts };
+enum Sp2Count { kSp2Asked, kSp2Retried, kSp2Unsettled, kSp2BatchAsked, kSp2BatchUnsettled, kSp2Squarings, kSp2Counts };
 void note_sp2(Sp2Count what, int by = 1);
 
 // An atom pair closer than the 7 Angstrom feather range, whose two-electron block is

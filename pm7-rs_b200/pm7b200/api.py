@@ -393,10 +393,11 @@ def launch_count():
 
 def sp2_counts():
     """SP2 purifications since process start and what became of them (`pm7_sp2_counts`)."""
-    out = (C.c_int64 * 5)()
+    out = (C.c_int64 * 6)()
     lib().pm7_sp2_counts.restype = None
     lib().pm7_sp2_counts(out)
-    return dict(zip(("asked", "retried", "unsettled", "batch_asked", "batch_unsettled"), (int(v) for v in out)))
+    names = ("asked", "retried", "unsettled", "batch_asked", "batch_unsettled", "squarings")
+    return dict(zip(names, (int(v) for v in out)))
 
 
 def profile_enable(on=True):
