@@ -367,7 +367,6 @@ static bool use_jacobi(int n) {
   return env && std::strcmp(env, "jacobi") == 0 && n <= kJacobiMax;
 }
 
-
 struct Diag {
   DeviceContext &ctx;
   cudaStream_t st;
@@ -673,7 +672,10 @@ struct Purifier {
 
 // The fp64 SP2 squarings run on the integer tensor cores (kernels_i8.cu) from kI8MinN orbitals
 // up, on the FP64 tensor cores in one cooperative launch below (kernels_sp2.cu);
-// PM7_SP2_GEMM=dmma|i8 forces one.
+// PM7_SP2_GEMM=dmma|i8 forces one. The line was drawn when the FP64 side was a launch per step (level
+// at ~600). A whole purification now takes, one launch against int8: 665 / 1,202 us at 768 orbitals,
+// 843 / 1,404 at 900, 1,129 / 1,486 at 1,026, 1,429 / 1,524 at 1,152, 1,871 / 1,719 at 1,218, 2,170 /
+// 1,697 at 1,344, 2,710 / 2,237 at 1,500: the two cross near 1,180, so the line lies too low.
 constexpr int kI8MinN = 768;
 static bool use_i8_sp2(int n) {
   const char *env = std::getenv("PM7_SP2_GEMM");
@@ -682,10 +684,6 @@ static bool use_i8_sp2(int n) {
   return n >= kI8MinN;
 }
 
-// Density solver for the SCF loop: SP2 above kJacobiMax orbitals (tensor-core squarings;
-// 16 against 37 ms per solve at 240 orbitals), the eigendecomposition (Diag) up to it and
-// when SP2 cannot settle. PM7_DENSITY_SOLVER=sp2|jacobi|syevd forces one (jacobi and syevd
-// turn SP2 off; syevd also keeps the final eigenvalues on cuSOLVER).
 // DIIS error below which the mixed-precision SCF switches to fp64 densities.
 static constexpr double kMixedSwitch = 1.0e-3;
 static constexpr double kMixedSwitchStep = 1.0e-6;  // rms density step that also ends the fp32 phase
@@ -697,6 +695,13 @@ static constexpr double kMixedSwitchStep = 1.0e-6;  // rms density step that als
 // cycle 6 and the SCF still ends at 17 from a clean history).
 static constexpr double kFock32Switch = 10.0;
 
+// Density solver for the SCF loop: SP2 above kJacobiMax orbitals, the eigendecomposition (Diag) up to
+// it and when SP2 cannot settle. PM7_DENSITY_SOLVER=sp2|jacobi|syevd forces one (jacobi and syevd turn
+// SP2 off; syevd also keeps the final eigenvalues on cuSOLVER). The line was drawn when a purification
+// was ~60 launches. A whole closed-shell solve now takes, dsyevd against sp2: 2.7 / 4.0 ms at 6
+// orbitals, 4.9 / 4.3 at 20, 5.5 / 5.4 at 32, 12.5 / 5.3 at 50, 14.1 / 5.5 at 62, 24.5 / 5.4 at 110: the
+// two cross near 20, so the line lies too high (up to it the SCF takes the reference's eigenvectors,
+// on exactly degenerate frontier levels too, where SP2 does not settle and is tried in vain).
 static bool use_sp2(int n) {
   const char *env = std::getenv("PM7_DENSITY_SOLVER");
   if (env && (std::strcmp(env, "syevd") == 0 || std::strcmp(env, "jacobi") == 0)) return false;

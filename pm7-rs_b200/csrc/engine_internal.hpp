@@ -256,9 +256,10 @@ struct EigvalsRequest {
 };
 // Eigenvalues only, many matrices at once (kernels_eig.cu): grouped by cluster size, one
 // tridiagonalisation and one Sturm launch per group; workspace from `scr` (grown in
-// stream order as needed). Every order must satisfy eigvals_supported(). whole_gpu: matrices from
-// kTriGridMin up are reduced one after the other by the whole GPU (kernels_trigrid.cu): for callers
-// that wait for them with nothing else to run; eigvals_check then reports an expired barrier after a
+// stream order as needed). Every order must satisfy eigvals_supported(). whole_gpu: matrices of order
+// 2 .. kTriGridMax are reduced one after the other by the whole GPU (kernels_trigrid.cu): for callers
+// that wait for them with nothing else to run (the levels of a single-molecule solve; the stage for
+// many matrices and the batch do not ask for it); eigvals_check then reports an expired barrier after a
 // stream synchronisation.
 void eigvals_device(cudaStream_t st, const std::vector<EigvalsRequest> &req, EigvalsScratch &scr,
                     bool whole_gpu = false);

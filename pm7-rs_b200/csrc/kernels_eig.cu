@@ -337,12 +337,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_tridiag(const EigvalsTask *__res
 }
 
 // Number of eigenvalues of the tridiagonal T = (d, e^2) below x, from the leading principal minors
-// of T - x: p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2}, a sign change per negative pivot
-// p_i / p_{i-1}. One dependent FMA per step where the pivots' recurrence (LAPACK dlaebz) needs a
+// of T - x (the Sturm sequence of Givens, with a running scale): p_i = (d_i - x) p_{i-1} - e_{i-1}^2
+// p_{i-2}, a sign change per negative pivot p_i / p_{i-1}. One dependent FMA per step where the pivots' recurrence (LAPACK dlaebz) needs a
 // division: the launch is a latency chain (14 warps an SM at 2,004 orbitals), 2.65 -> 1.17 ms there,
 // 0.27 -> 0.10 ms at 270. Each step perturbs d and e by a rounding, as the pivots do. The matrix is
-// scaled to elements of at most 2, so eight steps change the pair's scale by less than 1e256 and it
-// is renormalised (exactly) after each eight; a zero minor is a pivot of -1e-22.
+// scaled to elements of at most 2, so eight steps raise the pair's scale by less than 1e256 and it
+// is renormalised (exactly) after each eight; a zero minor is a pivot of -1e-22. Downwards there is no
+// such bound: over uncoupled zero rows (d = e = 0) and |x| < 1e-40 both minors reach zero within eight
+// steps and the rows after that count as negative, which moves the zero levels by 1e-40 at most.
 __device__ __forceinline__ int sturm_count(const double *__restrict__ d, const double *__restrict__ e2, int n,
                                            double x) {
   double p0 = 1.0, p1 = d[0] - x;

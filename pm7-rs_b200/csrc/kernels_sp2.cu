@@ -18,8 +18,8 @@
 // of 64), never on the grid, so the result has the same bits on every grid; products and sums
 // whose rounding decides a branch are written out, so that no contraction changes them.
 //
-// Measured (one purification of ~16 steps): n = 121 1.52 -> 0.15 ms (two spins 36 -> 14 ms a
-// solve), n = 204 0.73 -> 0.16, n = 270 1.10 -> 0.19, n = 666 1.36 -> 0.42 ms; a step 24 -> 5.3 us
+// Measured (one purification of ~16 steps, CUDA events around it in a solve): n = 121 0.18 ms (two spins
+// 36 -> 14 ms a solve), n = 204 0.73 -> 0.20, n = 310 0.26, n = 666 1.36 -> 0.50 ms; a step 24 -> 5.3 us
 // at n = 121, 54 -> 20 us at n = 666 (11 us of it DMMA issue), the Lanczos bounds 173 -> 70 us.
 #include <cuda_runtime.h>
 

@@ -14,9 +14,10 @@
 // Every sum is taken in a fixed order that depends on the matrix order alone, and a row's update is the
 // same operations wherever the row lies, so the values are the same bits on every grid.
 //
-// Measured: 0.66 ms at 204 orbitals (cluster kernel 1.7), 0.87 at 270 (3.1), 2.4 at 666 and 10.9 at
-// 2,004 (cuSOLVER dsyevd, values included, 7.4 and 25.7): 3.2 to 5.4 us a column, of which the
-// barrier is ~1 and the loads behind it ~0.5.
+// Measured (CUDA events): 0.39 ms at 121 orbitals, 0.65 at 204, 0.99 at 310, 2.4 at 666 and 11.1 at 2,004
+// (cuSOLVER dsyevd, values included, 7.4 and 25.7 at the last two): 3.2 to 5.5 us a column, of which the
+// barrier is ~1 and the loads behind it ~0.5. The levels of one matrix as a call with its copies, against
+// the cluster kernel: 0.80 / 2.2 ms at 204, 1.07 / 2.8 at 270, 2.2 / 6.1 at 512, 3.8 / 10.1 at 666.
 #include <cuda_runtime.h>
 
 #include <algorithm>
