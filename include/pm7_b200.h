@@ -280,6 +280,11 @@ pm7_status pm7_stage_sp2(int32_t n, const double *f, int32_t n_occ, double *p_ou
  * PM7_ERR_TIMEOUT, as pm7_run does when a wait expires; the CUDA context stays usable. */
 pm7_status pm7_stage_tf32_wait_drill(int32_t n);
 
+/* The same drill of the integer tensor-core squaring (65 <= n <= 4096; single CTAs or CTA pairs by
+ * the order): each CTA's copies stop after two stages, so that MMAs and copies have run when the
+ * waits expire, and the kernel waits for those before it leaves. */
+pm7_status pm7_stage_i8_wait_drill(int32_t n);
+
 /* Eigenvalues (ascending, no eigenvectors) of `count` symmetric matrices, the stage that
  * gives the reported MO energies when no orbitals are returned. Replaces the eigenvalue
  * half of `symmetric_eigen` (src/linalg.rs:231-278, faer self_adjoint_eigen) as used by

@@ -2078,6 +2078,39 @@ pm7_status pm7_stage_sp2_step_i8(int32_t n, const double *x, int32_t square, dou
   });
 }
 
+pm7_status pm7_stage_i8_wait_drill(int32_t n) {
+  return guarded([&] {
+    if (n < 65 || n > 4096) throw Failure{PM7_ERR_INVALID_INPUT, "wait drill needs 65 <= n <= 4096"};
+    DeviceContext &ctx = context_for(0);
+    std::lock_guard<std::mutex> lock(ctx.run_mutex);
+    CUDA_OK(cudaSetDevice(ctx.device));
+    cudaStream_t st = ctx.stream;
+    const size_t nn = (size_t)n * n;
+    DevBuf<double> X, Y, state, parts;
+    DevBuf<int8_t> dig0, dig1;
+    DevBuf<int> err;
+    for (DevBuf<double> *b : {&X, &Y}) {
+      b->alloc(nn, st);
+      CUDA_OK(cudaMemsetAsync(b->p, 0, sizeof(double) * nn, st));
+    }
+    for (DevBuf<int8_t> *d : {&dig0, &dig1}) {
+      d->alloc(sp2_i8_digit_bytes(n), st);
+      CUDA_OK(cudaMemsetAsync(d->p, 0, sp2_i8_digit_bytes(n), st));
+    }
+    state.alloc(kSp2Len, st);
+    parts.alloc(2 * (size_t)sp2_i8_tiles(n), st);
+    err.alloc(1, st);
+    CUDA_OK(cudaMemsetAsync(err.p, 0, sizeof(int), st));
+    launch_sp2_reset(st, state.p);
+    launch_sp2_step_i8(st, n, dig0.p, X.p, Y.p, dig1.p, state.p, parts.p, 0, err.p, 2);
+    int e = 0;
+    CUDA_OK(cudaMemcpyAsync(&e, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CUDA_OK(cudaStreamSynchronize(st));
+    CUDA_OK(cudaGetLastError());
+    if (e) throw Failure{PM7_ERR_TIMEOUT, "tcgen05 i8 squaring: a pipeline wait expired (drill)"};
+  });
+}
+
 pm7_status pm7_stage_sp2(int32_t n, const double *f, int32_t n_occ, double *p_out, double info[6]) {
   return guarded([&] {
     if (n < 1 || n_occ < 0 || n_occ > n || !f || !p_out || !info)

@@ -198,8 +198,10 @@ size_t sp2_i8_digit_bytes(int n);
 int sp2_i8_tiles(int n);
 void launch_sp2_digits(cudaStream_t st, int n, const double *X, int8_t *dig, const double *state, int step,
                        int *error);
+// withhold: the failure drill, a CTA's copies from that stage on never come, so that the pipeline's waits
+// run out.
 void launch_sp2_step_i8(cudaStream_t st, int n, const int8_t *dig, const double *x_in, double *x_out, int8_t *dig_out,
-                        double *state, double *parts, int step, int *error);
+                        double *state, double *parts, int step, int *error, int withhold = 1 << 30);
 }  // namespace pm7
 
 namespace pm7 {

@@ -60,7 +60,7 @@ constexpr int kA1 = 2 * kHalf, kB0 = 4 * kHalf, I_STAGE = 6 * kHalf;
 template <int ST, int W>
 struct I8Shape {
   static constexpr int STAGES = ST, WIDTH = W, LDT = W + 1;
-  static constexpr int SMEM = ST * I_STAGE + IM * LDT * 8 + 128 + (3 * ST + 2) * 8 + 16 + 1024;
+  static constexpr int SMEM = ST * I_STAGE + IM * LDT * 8 + 128 + (3 * ST + 3) * 8 + 16 + 1024;
   static_assert(SMEM <= 227 * 1024, "one CTA per SM within the shared-memory limit");
 };
 using OneShape = I8Shape<3, 64>;   // one pass: the 64 columns of a tile at once
@@ -275,9 +275,10 @@ template <class Shape>
 struct I8Smem {
   unsigned char *stage;
   double *T, *red;
-  uint64_t *full, *empty, *peer, *tmem_full, *tmem_empty;
+  uint64_t *full, *empty, *peer, *tmem_full, *tmem_empty, *drained;
   uint32_t *tmem_slot;
   volatile int *abort_flag;
+  int *fills;  // stages handed to the copies (the producer's last word)
   __device__ explicit I8Smem(unsigned char *raw) {
     stage = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
     T = reinterpret_cast<double *>(stage + Shape::STAGES * I_STAGE);
@@ -287,8 +288,10 @@ struct I8Smem {
     peer = empty + Shape::STAGES;
     tmem_full = peer + Shape::STAGES;
     tmem_empty = tmem_full + 1;
-    tmem_slot = reinterpret_cast<uint32_t *>(tmem_empty + 1);
+    drained = tmem_empty + 1;
+    tmem_slot = reinterpret_cast<uint32_t *>(drained + 1);
     abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    fills = reinterpret_cast<int *>(tmem_slot + 2);
   }
 };
 
@@ -300,7 +303,8 @@ struct I8Smem {
 __global__ void __launch_bounds__(192, 1) k_sp2_step_i8(const int8_t *__restrict__ dig, int n,
                                                         const double *__restrict__ x_in, double *__restrict__ x_out,
                                                         double *__restrict__ state, int step,
-                                                        double *__restrict__ parts, int *__restrict__ error) {
+                                                        double *__restrict__ parts, int *__restrict__ error,
+                                                        int withhold) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   if (!sp2_active(state, step)) return;  // the whole CTA, before any barrier or TMEM set-up
   const int tiles = i8_tile_count(n);
@@ -318,6 +322,7 @@ __global__ void __launch_bounds__(192, 1) k_sp2_step_i8(const int8_t *__restrict
     }
     mbar_init(S.tmem_full, 1);
     mbar_init(S.tmem_empty, 4);  // one arrival per epilogue warp
+    mbar_init(S.drained, 1);
     *S.abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -347,11 +352,13 @@ __global__ void __launch_bounds__(192, 1) k_sp2_step_i8(const int8_t *__restrict
           const uint32_t st = smem_u32(S.stage + s * I_STAGE);
           const int8_t *b = dig + block_at(bn >> 1, kt, 0, kts) + kHalf * (bn & 1);
           mbar_expect_tx(&S.full[s], I_STAGE);
+          if (g >= withhold) continue;  // failure drill: the stage never fills, every wait runs out
           load_block(st, dig + block_at(bm, kt, 0, kts), 2 * kBlock, &S.full[s]);
           load_block(st + kB0, b, kHalf, &S.full[s]);
           load_block(st + kB0 + kHalf, b + kBlock, kHalf, &S.full[s]);
         }
       }
+      *S.fills = g;
     }
   } else if (warp == 5) {
     if (lane == 0) {  // MMA issuer: digit pairs (i, j), i + j <= 7, into accumulator i + j
@@ -428,6 +435,14 @@ __global__ void __launch_bounds__(192, 1) k_sp2_step_i8(const int8_t *__restrict
   if (threadIdx.x == 0 && *S.abort_flag) atomicExch(error, 1);
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
+  if (*S.abort_flag) {
+    if (warp == 4 && lane == 0) drain_ring(S.full, *S.fills, ISTAGES);
+    if (warp == 5 && lane == 0) {
+      mma_commit(S.drained);
+      mbar_drain(S.drained, 0u);
+    }
+    __syncthreads();
+  }
   if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
@@ -492,7 +507,7 @@ __device__ __forceinline__ void arrive_leader(uint64_t *bar) {
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1)
     k_sp2_step_i8_pair(const int8_t *__restrict__ dig, int n, const double *__restrict__ x_in,
                        double *__restrict__ x_out, double *__restrict__ state, int step, double *__restrict__ parts,
-                       int *__restrict__ error) {
+                       int *__restrict__ error, int withhold) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   if (!sp2_active(state, step)) return;  // the whole cluster, before any barrier or TMEM set-up
   const int tiles = pair_tile_count(n);
@@ -512,6 +527,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1)
     }
     mbar_init(S.tmem_full, 1);
     mbar_init(S.tmem_empty, 16);  // one arrival per epilogue warp of both CTAs
+    mbar_init(S.drained, 1);
     *S.abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -527,7 +543,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1)
   const uint32_t tmem = *S.tmem_slot;
 
   if (warp == 8) {
-    if (lane == 0) {  // producer: this CTA's 128 rows of A and 64 rows of B, counted on the leader's barriers
+    if (lane == 0) {  // producer: this CTA's 128 rows of A and 64 rows of B, counted on its own barriers
       int g = 0;
       bool ok = true;
       for (int t = first; t < tiles && ok; t += stride) {
@@ -556,6 +572,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1)
             two = kt + 1 < kts;
           }
           mbar_expect_tx(&S.full[s], two ? I_STAGE : I_STAGE / 2);
+          if (g >= withhold) continue;  // (see k_sp2_step_i8)
           load_block(st, a, kBlock, &S.full[s]);
           load_block(st + kB0, b, kHalf, &S.full[s]);
           if (two) {
@@ -564,6 +581,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1)
           }
         }
       }
+      *S.fills = g;
     }
   } else if (warp == 9) {
     if (lane == 0 && rank == 1) {  // tells the leader of each stage that this CTA has filled
@@ -705,6 +723,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1)
   if (threadIdx.x == 0 && *S.abort_flag) atomicExch(error, 1);
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
+  if (*S.abort_flag) {
+    if (warp == 8 && lane == 0) drain_ring(S.full, *S.fills, ISTAGES);
+    if (warp == 9 && lane == 0 && rank == 0) {  // (the leader alone issues MMAs)
+      // (on this CTA's barrier alone: an arrival on its way to the other might find it gone)
+      asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(S.drained))
+                   : "memory");
+      mbar_drain(S.drained, 0u);
+    }
+    __syncthreads();
+  }
   // the pair leaves together: neither CTA's barriers, shared memory or TMEM are in use any more
   asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
   if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
@@ -799,13 +827,14 @@ void launch_sp2_digits(cudaStream_t st, int n, const double *X, int8_t *dig, con
 // 6,000. While one wave holds them the single CTAs are faster: they share a product among twice as
 // many SMs (89 against 113 us at 1,400, 71 against 90 at 1,000).
 void launch_sp2_step_i8(cudaStream_t st, int n, const int8_t *dig, const double *x_in, double *x_out, int8_t *dig_out,
-                        double *state, double *parts, int step, int *error) {
+                        double *state, double *parts, int step, int *error, int withhold) {
   const I8Limits L = i8_limits();
   if (i8_tile_count(n) > L.sms)
     k_sp2_step_i8_pair<<<2 * std::min(L.pairs, pair_tile_count(n)), 320, PairShape::SMEM, st>>>(dig, n, x_in, x_out, state, step,
-                                                                                       parts, error);
+                                                                                       parts, error, withhold);
   else
-    k_sp2_step_i8<<<std::min(L.sms, i8_tile_count(n)), 192, OneShape::SMEM, st>>>(dig, n, x_in, x_out, state, step, parts, error);
+    k_sp2_step_i8<<<std::min(L.sms, i8_tile_count(n)), 192, OneShape::SMEM, st>>>(dig, n, x_in, x_out, state, step, parts, error,
+                                                                               withhold);
   note_launch();
   launch_sp2_digits(st, n, x_out, dig_out, state, step, error);
 }

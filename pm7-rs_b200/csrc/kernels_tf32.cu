@@ -76,7 +76,8 @@ __device__ __forceinline__ void product_tile(int bm, int bn, const CUtensorMap *
   uint64_t *full = reinterpret_cast<uint64_t *>(smem + STAGES * STAGE_BYTES);
   uint64_t *empty = full + STAGES;
   uint64_t *done = empty + STAGES;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
+  uint64_t *drained = done + 1;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drained + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int m0 = bm * TM, n0 = bn * TN;
@@ -89,6 +90,7 @@ __device__ __forceinline__ void product_tile(int bm, int bn, const CUtensorMap *
       mbar_init(&empty[s], 1);
     }
     mbar_init(done, 1);
+    mbar_init(drained, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -102,12 +104,14 @@ __device__ __forceinline__ void product_tile(int bm, int bn, const CUtensorMap *
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = *tmem_slot;
 
+  int fills = 0;  // stages handed to the copies (the producer)
   if (warp == 0 && lane == 0) {
     // producer: TMA ring
     for (int kt = 0; kt < ktiles; ++kt) {
       const int s = kt % STAGES;
       if (kt >= STAGES && !mbar_wait(&empty[s], (uint32_t)((kt / STAGES - 1) & 1), abort_flag)) break;
       unsigned char *st = smem + s * STAGE_BYTES;
+      fills = kt + 1;
       mbar_expect_tx(&full[s], STAGE_BYTES);
       if (withhold_copies) continue;  // failure drill: the stage never fills, every wait runs out
       const int k0 = kt * TK;
@@ -178,6 +182,14 @@ __device__ __forceinline__ void product_tile(int bm, int bn, const CUtensorMap *
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
+  if (*abort_flag) {
+    if (warp == 0 && lane == 0) drain_ring(full, fills, STAGES);
+    if (warp == 1 && lane == 0) {
+      mma_commit(drained);
+      mbar_drain(drained, 0u);
+    }
+    __syncthreads();
+  }
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TN));
 }
 

@@ -57,6 +57,31 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
   return false;
 }
 
+// After an expired wait: what this CTA still has in flight is waited for, again with a limit and without
+// a look at the abort flag, so that no copy lands in shared memory that the CTA has given back and no
+// MMA reads it or writes tensor memory that has been freed.
+constexpr unsigned long long kDrainNs = 100000000ull;  // 0.1 s per barrier
+__device__ __forceinline__ void mbar_drain(uint64_t *bar, uint32_t parity) {
+  const uint32_t addr = smem_u32(bar);
+  const unsigned long long t0 = global_ns();
+  for (uint32_t it = 0; it < (1u << 30); ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (done || ((it & 15) == 15 && global_ns() - t0 > kDrainNs)) return;
+  }
+}
+// The copies of a ring that has been filled `fills` times (one thread).
+__device__ __forceinline__ void drain_ring(uint64_t *full, int fills, int stages) {
+  for (int k = fills > stages ? fills - stages : 0; k < fills; ++k)
+    mbar_drain(&full[k % stages], (uint32_t)((k / stages) & 1));
+}
+
 __device__ __forceinline__ void tma_load_2d(void *smem_dst, const CUtensorMap *map, uint64_t *bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(

@@ -27,7 +27,8 @@ EXPORTED = [
     "pm7_correction_gradient", "pm7_run_batch_gradient", "pm7_engine_submit_gradient",
     "pm7_dandc_options_default", "pm7_run_dandc", "pm7_dandc_result_free", "pm7_stage_dandc_partition",
     "pm7_dandc_abi_sizes", "pm7_stage_seqsum", "pm7_stage_tf32_wait_drill",
-    "pm7_engine_stats", "pm7_stage_fock_fp32", "pm7_stage_sp2_step_i8",
+    "pm7_engine_stats", "pm7_stage_fock_fp32", "pm7_stage_sp2_step_i8", "pm7_stage_i8_wait_drill",
+    "pm7_stage_sp2", "pm7_stage_levels", "pm7_sp2_counts",
 ]
 
 
@@ -341,6 +342,11 @@ def tf32_wait_drill(n=128):
     """Status code of the bounded-wait drill (pm7_stage_tf32_wait_drill): the tcgen05
     squaring with its copies withheld; 10 (PM7_ERR_TIMEOUT) when every wait gave up."""
     return int(lib().pm7_stage_tf32_wait_drill(int(n)))
+
+
+def i8_wait_drill(n):
+    """The same drill of the integer tensor-core squaring (pm7_stage_i8_wait_drill)."""
+    return int(lib().pm7_stage_i8_wait_drill(C.c_int32(int(n))))
 
 
 def seqsum(a, b=None, device=0):
