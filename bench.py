@@ -167,8 +167,13 @@ def fp64_dgemm_peak(device):
     return best
 
 
-def read_traffic(kernel):
-    """Per-launch DRAM bytes of `kernel` from a committed ncu summary, scaled to the bench size."""
+TRAFFIC_NAO = 2004  # the order that the committed summaries were captured at
+
+
+def read_traffic(kernel, nao):
+    """Per-launch DRAM bytes of `kernel` from a committed ncu summary; None at any other order."""
+    if nao != TRAFFIC_NAO:
+        return None
     p = ROOT / "profiles" / "traffic.txt"
     if not p.exists():
         return None
@@ -392,7 +397,7 @@ def run_b200(args, world, rank, local):
         flops = (squarings if sq_calls else 0) * float(nao) ** 3 + cm_calls * 2.0 * float(nao) ** 3  # algorithmic
         launches_g = sq_calls + cm_calls
         achieved = flops / (gemm_ms * 1e-3) / 1e12
-        traffic = None if sq_calls else read_traffic("commutator_gemm")  # (captured at nao 2,004)
+        traffic = None if sq_calls else read_traffic("commutator_gemm", nao)
         label = ("k_sp2_purify (a purification per launch) + k_gemm_tn (F.P)" if sq_calls else "k_gemm_tn (F.P)") + \
             ", FP64 DMMA mma.sync.m16n8k8"
         roofline = {"kernel": label, "bound": "tensor", "achieved": achieved,
@@ -418,7 +423,7 @@ def run_b200(args, world, rank, local):
                               "squares, tcgen05.mma kind::i8 on int8 digit planes by bulk copies, TMEM; fp64 accuracy "
                               "by the Ozaki scheme", "bound": "tensor", "achieved": achieved_tops,
                     "peak": peak_i8, "unit": "TOP/s", "frac": achieved_tops / peak_i8,
-                    "traffic": read_traffic("sp2_square_i8"), "launches": i8_calls, "ms_avg": ms_avg,
+                    "traffic": read_traffic("sp2_square_i8", nao), "launches": i8_calls, "ms_avg": ms_avg,
                     "algorithmic_per_launch": f"{ops:.4g} int8 ops ({float(nao) ** 3:.4g} fp64-equivalent flop)",
                     "fp64_equivalent_tflops": fp64_eq, "fp64_equivalent_frac_of_dgemm": (fp64_eq / dgemm) if dgemm else None,
                     "peak_source": "twice the measured bf16 dense rate in MEASURED_PEAKS.json"}
@@ -443,7 +448,7 @@ def run_b200(args, world, rank, local):
         achieved_gbs = nbytes / (fock_ms / fock_calls * 1e-3) / 1e9
         fock_roof = {"kernel": "fock (k_fock_far + k_fock_near + k_fock_atom)", "bound": "hbm",
                      "achieved": achieved_gbs, "peak": peaks.get("hbm_gbs"), "unit": "GB/s",
-                     "frac": achieved_gbs / peaks.get("hbm_gbs", 6650.0), "traffic": read_traffic("fock"),
+                     "frac": achieved_gbs / peaks.get("hbm_gbs", 6650.0), "traffic": read_traffic("fock", nao),
                      "algorithmic_per_launch": f"{nbytes:.4g} B", "peak_source": "MEASURED_PEAKS.json hbm_gbs"}
     # whole-solve roofline: iterations x (Fock bytes / HBM + dense flops / FP64 peak), the
     # dense flops per iteration being an eigensolve (10/3 n^3), the density (n^2 n_occ) and the

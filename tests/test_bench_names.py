@@ -22,3 +22,10 @@ def test_every_kernel_bench_names_exists():
     named = set(re.findall(r"\bk_[a-z0-9_]+", (ROOT / "bench.py").read_text()))
     defined = set(re.findall(r"\b(k_[a-z0-9_]+)\s*\(", SOURCES))
     assert named and not named - defined, named - defined
+
+
+def test_traffic_is_given_at_the_order_it_was_captured_at():
+    import bench
+
+    assert bench.read_traffic("fock", bench.TRAFFIC_NAO) > 0
+    assert bench.read_traffic("fock", 6000) is None
