@@ -289,7 +289,7 @@ pm7_status pm7_stage_i8_wait_drill(int32_t n);
  * gives the reported MO energies when no orbitals are returned. Replaces the eigenvalue
  * half of `symmetric_eigen` (src/linalg.rs:231-278, faer self_adjoint_eigen) as used by
  * run_pm7's final step (src/scf.rs:1299-1305). Matrices are packed row-major one after
- * another (orders[i]^2 doubles each; order <= 8192), eigenvalues likewise (orders[i]
+ * another (orders[i]^2 doubles each; order <= 4096), eigenvalues likewise (orders[i]
  * each). Host buffers; runs on `device`. */
 pm7_status pm7_stage_eigenvalues(int32_t count, const int32_t *orders, const double *a, double *w,
                                  int32_t device);
