@@ -704,6 +704,7 @@ __global__ void __launch_bounds__(GT) k_sp2_purify(Sp2GridArgs A) {
     }
     __syncthreads();
     if (late) {
+      if (warp >= 12) asm volatile("cp.async.wait_all;" ::: "memory");  // no copy outlives the CTA
       if (threadIdx.x == 0) atomicExch(A.error, 1);
       return;
     }
